@@ -19,16 +19,17 @@
 // streams, or different host threads without ordering) race and corrupt each
 // other.
 //
-// The kernels are the one-warp-per-row form of the plain minibatch kernel:
-// attractive pass in CSR order, repulsive pass over the minibatch's negatives
-// (cpp/algo/algo.hpp:521-584, 586-649), result staged, then committed to x by a
-// second launch (algo.hpp:651-666), so every read in the first launch sees the
-// pre-minibatch values as the reference's does.
+// A row's attractive pass in CSR order and its repulsive pass over the minibatch's
+// negatives (cpp/algo/algo.hpp:521-584, 586-649) are spread over the warps of one
+// CTA, the result is staged and committed to x by a second launch
+// (algo.hpp:651-666), so every read in the first launch sees the pre-minibatch
+// values as the reference's does.
 #include <cuda_runtime.h>
 
 #include <string>
 
 #include "../../include/distembed_gb300.h"
+#include "de_device.cuh"
 
 namespace de {
 void set_thread_error(const std::string &msg);  // de_runtime.cpp
@@ -61,66 +62,143 @@ struct NoAllocArgs {
 
 __device__ __forceinline__ float nclip(float v, float b) { return v > b ? b : (v < -b ? -b : v); }
 
-__device__ __forceinline__ float nwarp_sum(float v) {
+// Components of a row held by a lane: with wide loads (x 16-byte aligned, so every
+// row is) dev::Frag's, else l, l + 32, ... by 4-byte loads.
+template <int D, bool kWide>
+__device__ __forceinline__ void nload(de::dev::Frag<D> &f, const float *row, int lane) {
+  if constexpr (kWide) {
+    de::dev::load_nc(f, row, lane);
+  } else {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
-  return v;
+    for (int t = 0; t < D / 32; ++t) f.v[t] = __ldg(row + lane + 32 * t);
+  }
 }
 
-// One row per warp; lane l holds components l, l+32, ... of the row.
-template <int D, bool kAttract>
-__device__ __forceinline__ double nforce(float (&acc)[D / 32], const float (&xi)[D / 32], const float *xn_row,
-                                         float lr, float bound, int lane) {
-  constexpr int N = D / 32;
-  float diff[N];
-  float part = 0.f;
+// The pairs of x_i with up to U rows (lane u of `ids`: row u, -1 = none), all
+// loads issued before the first is used; the U squared distances are reduced
+// together (multi_warp_sum), so a lane divides for one pair.
+template <int D, int U, bool kWide, bool kAttract>
+__device__ __forceinline__ void nforces(const NoAllocArgs &a, de::dev::Frag<D> &acc, const de::dev::Frag<D> &xi,
+                                        int ids, bool want_loss, double &loss, int lane) {
+  constexpr int N = D / 32, L = de::dev::Log2<U>::value;
+  de::dev::Frag<D> xn[U];
+  unsigned mask = 0;
 #pragma unroll
-  for (int t = 0; t < N; ++t) {
-    diff[t] = xi[t] - __ldg(xn_row + lane + 32 * t);
-    part = fmaf(diff[t], diff[t], part);
-  }
-  const float r = nwarp_sum(part);
-  const float c = kAttract ? -2.0f / (1.0f + r) : 2.0f / ((r + 1e-6f) * (1.0f + r));
-#pragma unroll
-  for (int t = 0; t < N; ++t) acc[t] = fmaf(lr, nclip(diff[t] * c, bound), acc[t]);
-  return kAttract ? double(log1pf(r)) : double(logf((1.0f + r) / (r + 1e-6f)));
-}
-
-template <int D>
-__global__ void __launch_bounds__(256) noalloc_rows_kernel(const NoAllocArgs a) {
-  constexpr int N = D / 32;
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (r >= a.rows) return;
-  const int row = a.base + r;
-  float xi[N], acc[N];
-#pragma unroll
-  for (int t = 0; t < N; ++t) {
-    xi[t] = __ldg(a.x + size_t(row) * D + lane + 32 * t);
-    acc[t] = 0.f;
-  }
-  double loss = 0.0;
-  for (int e = __ldg(a.rowptr + row), e1 = __ldg(a.rowptr + row + 1); e < e1; ++e) {
-    const int nb = __ldg(a.col + e);
-    if (nb == a.skip) continue;
-    loss += nforce<D, true>(acc, xi, a.x + size_t(nb) * D, a.lr, a.bound, lane);
-  }
-  if (r < a.rep_rows)
-    for (int k = 0; k < a.ns; ++k) {
-      const int nb = __ldg(a.negs + k);
-      if (nb < 0 || nb >= a.n) continue;  // a draw equal to n contributes nothing
-      loss += nforce<D, false>(acc, xi, a.x + size_t(nb) * D, a.lr, a.bound, lane);
+  for (int u = 0; u < U; ++u) {
+    const int nb = __shfl_sync(kFullMask, ids, u);
+    if (nb >= 0) {
+      nload<D, kWide>(xn[u], a.x + size_t(nb) * D, lane);
+      mask |= 1u << u;
+    } else {
+      xn[u] = xi;
     }
+  }
+  if (mask == 0) return;
+  float p[U];
 #pragma unroll
-  for (int t = 0; t < N; ++t) a.staged[size_t(r) * D + lane + 32 * t] = xi[t] + acc[t];
-  if (lane == 0) a.partial[r] = loss;
+  for (int u = 0; u < U; ++u) {
+    p[u] = 0.f;
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      xn[u].v[t] = xi.v[t] - xn[u].v[t];
+      p[u] = fmaf(xn[u].v[t], xn[u].v[t], p[u]);
+    }
+  }
+  const float r = de::dev::multi_warp_sum<U>(p, lane);
+  const int v = (lane >> (5 - L)) & (U - 1);
+  float c = kAttract ? -2.0f / (1.0f + r) : 2.0f / ((r + 1e-6f) * (1.0f + r));
+  if (!((mask >> v) & 1u)) c = 0.f;
+  else if (want_loss && (lane & ((32 >> L) - 1)) == 0)
+    loss += kAttract ? double(log1pf(r)) : double(logf((1.0f + r) / (r + 1e-6f)));
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const float cu = __shfl_sync(kFullMask, c, u << (5 - L));
+#pragma unroll
+    for (int t = 0; t < N; ++t) acc.v[t] = fmaf(a.lr, nclip(xn[u].v[t] * cu, a.bound), acc.v[t]);
+  }
 }
 
-template <int D>
-__global__ void __launch_bounds__(256) noalloc_commit_kernel(const NoAllocArgs a) {
-  const int64_t total = int64_t(a.rows) * D;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x)
-    a.x[size_t(a.base) * D + i] = a.staged[i];
+// One row per CTA of W warps: the row's CSR entries and then its negatives in
+// groups of U, group q on warp q % W; the warps' sums are added in warp order.
+// A minibatch is too small to fill the GPU with bytes, so a call takes as long as
+// the longest chain of dependent loads.  Here a row of up to 8 W pairs is one
+// round: row pointer, column ids, rows.  Measured on the epoch of a 2,000-vertex
+// kNN graph (8 calls of 256 rows of about 14 neighbours, dim 64, 5 negatives):
+// 305 us with a warp per row and one neighbour in flight, 52 us so (6.5 us a call,
+// both launches in it).
+template <int D, int U, int W, bool kWide>
+__global__ void __launch_bounds__(W * 32) noalloc_rows_kernel(const NoAllocArgs a) {
+  constexpr int N = D / 32;
+  __shared__ float sums[W][D];
+  __shared__ double losses[W];
+  de::dev::pdl_wait();
+  de::dev::pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x, row = a.base + r;
+  const int e0 = __ldg(a.rowptr + row), deg = __ldg(a.rowptr + row + 1) - e0;
+  de::dev::Frag<D> xi, acc;
+  nload<D, kWide>(xi, a.x + size_t(row) * D, lane);
+  acc.zero();
+  const bool want_loss = a.loss != nullptr;
+  double loss = 0.0;
+  const int ge = (deg + U - 1) / U;
+  const int groups = ge + (r < a.rep_rows ? (a.ns + U - 1) / U : 0);
+  for (int q = warp; q < groups; q += W) {
+    if (q < ge) {
+      const int k = q * U + lane;
+      int id = lane < U && k < deg ? __ldg(a.col + e0 + k) : -1;
+      if (id == a.skip) id = -1;
+      nforces<D, U, kWide, true>(a, acc, xi, id, want_loss, loss, lane);
+    } else {
+      const int k = (q - ge) * U + lane;
+      int id = lane < U && k < a.ns ? __ldg(a.negs + k) : -1;
+      if (id >= a.n) id = -1;  // a draw equal to n contributes nothing
+      nforces<D, U, kWide, false>(a, acc, xi, id, want_loss, loss, lane);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < N; ++t) sums[warp][t * 32 + lane] = acc.v[t];
+  if (want_loss) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(kFullMask, loss, o);
+    if (lane == 0) losses[warp] = loss;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  acc.zero();
+#pragma unroll
+  for (int w = 0; w < W; ++w)
+#pragma unroll
+    for (int t = 0; t < N; ++t) acc.v[t] += sums[w][t * 32 + lane];
+#pragma unroll
+  for (int t = 0; t < N; ++t) acc.v[t] = xi.v[t] + acc.v[t];
+  if constexpr (kWide) {
+    de::dev::store<D, false>(acc, a.staged + size_t(r) * D, lane);
+  } else {
+#pragma unroll
+    for (int t = 0; t < N; ++t) a.staged[size_t(r) * D + lane + 32 * t] = acc.v[t];
+  }
+  if (want_loss && lane == 0) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) s += losses[w];
+    a.partial[r] = s;
+  }
+}
+
+// x rows = staged rows, and the minibatch's loss.  Bound by its launch: 64 KB at
+// 256 rows, dim 64.
+template <bool kWide>
+__global__ void __launch_bounds__(256) noalloc_commit_kernel(const NoAllocArgs a, int64_t total, int64_t first) {
+  de::dev::pdl_trigger();
+  de::dev::pdl_wait();
+  const int64_t i0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, step = int64_t(gridDim.x) * blockDim.x;
+  if constexpr (kWide) {
+    for (int64_t i = i0; i < total / 4; i += step)
+      reinterpret_cast<float4 *>(a.x + first)[i] = reinterpret_cast<const float4 *>(a.staged)[i];
+  } else {
+    for (int64_t i = i0; i < total; i += step) a.x[first + i] = a.staged[i];
+  }
   if (blockIdx.x != 0 || a.loss == nullptr) return;
   __shared__ double red[256];
   double s = 0.0;
@@ -132,6 +210,38 @@ __global__ void __launch_bounds__(256) noalloc_commit_kernel(const NoAllocArgs a
     __syncthreads();
   }
   if (threadIdx.x == 0) *a.loss = red[0];
+}
+
+// Both kernels are launched with a programmatic dependency on the kernel before
+// them in the stream: each waits for that kernel's end before it reads anything
+// (griddepcontrol.wait comes first), so only its launch overlaps.
+template <typename... P, typename... A>
+cudaError_t nlaunch(void (*k)(P...), int grid, int block, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+// Eight warps a row where the rows then still fit the GPU at once (152 SMs x 8
+// CTAs of 256 threads), so that the longest rows finish sooner; four beyond.
+constexpr int kWideTeamRows = 152 * 8;
+
+template <int D, bool kWide>
+cudaError_t nrun(const NoAllocArgs &a, cudaStream_t s) {
+  constexpr int U = D == 256 ? 4 : 8;
+  cudaError_t e = a.rows <= kWideTeamRows ? nlaunch(noalloc_rows_kernel<D, U, 8, kWide>, a.rows, 256, s, a)
+                                          : nlaunch(noalloc_rows_kernel<D, U, 4, kWide>, a.rows, 128, s, a);
+  if (e != cudaSuccess) return e;
+  const int64_t total = int64_t(a.rows) * D, per = 256 * (kWide ? 4 : 1);
+  const int grid = int((total + per - 1) / per < 152 * 4 ? (total + per - 1) / per : 152 * 4);
+  return nlaunch(noalloc_commit_kernel<kWide>, grid, 256, s, a, total, int64_t(a.base) * D);
 }
 
 // Device address of the scratch array in the current device's context.  It is
@@ -194,15 +304,15 @@ extern "C" int de_minibatch_noalloc(int64_t n, const int32_t *rowptr, const int3
   a.partial = reinterpret_cast<double *>(static_cast<unsigned char *>(scratch) + kNoAllocMaxRowFloats * sizeof(float));
   a.loss = loss;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int grid_rows = int((rows + 7) / 8);
-  const int grid_commit = int((rows * dim + 255) / 256 < 152 * 4 ? (rows * dim + 255) / 256 : 152 * 4);
+  // wide loads and stores need x on a 16-byte boundary; a caller's x need not be
+  const bool wide = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  cudaError_t e = cudaSuccess;
   switch (dim) {
-    case 32: noalloc_rows_kernel<32><<<grid_rows, 256, 0, s>>>(a); noalloc_commit_kernel<32><<<grid_commit, 256, 0, s>>>(a); break;
-    case 64: noalloc_rows_kernel<64><<<grid_rows, 256, 0, s>>>(a); noalloc_commit_kernel<64><<<grid_commit, 256, 0, s>>>(a); break;
-    case 128: noalloc_rows_kernel<128><<<grid_rows, 256, 0, s>>>(a); noalloc_commit_kernel<128><<<grid_commit, 256, 0, s>>>(a); break;
-    default: noalloc_rows_kernel<256><<<grid_rows, 256, 0, s>>>(a); noalloc_commit_kernel<256><<<grid_commit, 256, 0, s>>>(a); break;
+    case 32: e = wide ? nrun<32, true>(a, s) : nrun<32, false>(a, s); break;
+    case 64: e = wide ? nrun<64, true>(a, s) : nrun<64, false>(a, s); break;
+    case 128: e = wide ? nrun<128, true>(a, s) : nrun<128, false>(a, s); break;
+    default: e = wide ? nrun<256, true>(a, s) : nrun<256, false>(a, s); break;
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     de::set_thread_error(std::string("de_minibatch_noalloc launch: ") + cudaGetErrorString(e));
     return DE_ERR_CUDA;
