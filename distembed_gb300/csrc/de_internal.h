@@ -71,7 +71,6 @@ struct Schedule {
   std::vector<int32_t> n_parts;    // partial slots used by batch j
   std::vector<int32_t> n_split;    // arrival counters used by batch j
   int max_parts = 0, max_split = 0;
-  std::vector<int64_t> cta_off;    // [batches + 1] CTA counts (prefix) of the minibatch launches
   WorkItem *d_items = nullptr;
   int64_t n_items = 0;
 };
@@ -214,7 +213,8 @@ int copy_loss(de_handle *h, double *out, int32_t epochs);
 
 // Launchers (de_plain.cu).  pdl: launch with a programmatic dependency on the
 // previous kernel in the stream.
-cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, int grid, bool pdl, cudaStream_t s);
+// teams: several warps to a work item where plain_team_warps says so (one otherwise).
+cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, bool teams, bool pdl, cudaStream_t s);
 cudaError_t launch_flush(int dim, const FlushArgs &a, bool pdl, cudaStream_t s);
 cudaError_t launch_spmm(int dim, const SpmmArgs &a, cudaStream_t s);
 
@@ -237,6 +237,19 @@ cudaError_t launch_f32_to_f64(const float *src, double *dst, int64_t count, cuda
 constexpr int kPlainWarps = 4;      // warps per CTA of the plain batch kernel
 constexpr int kPlainMinBlocks = 8;  // resident CTAs per SM the register budget targets (one wave of
                                     // work items at minibatch 4096: 152 x 8 x 4 warps)
+// Warps to a work item of the FP32 plain form.  Several shorten the chain of a row
+// as long as the minibatch's warps then still run at once (152 SMs x 32 resident
+// warps, 16 at dim 256).  Measured crossings, in items of a minibatch: four against
+// two warps at 800 to 1,000 for every dim (kNN-20k, dim 128: 540 items 4.5 against
+// 5.2 us, 1,080 items 6.2 against 6.5, at dim 64 5.8 against 5.6); two against one
+// at about 2,500 (2,150 items 7.9 against 9.1 us, 3,200 items 11.1 against 10.5) and
+// at dim 256 at 1,600 to 2,000 (1,600 items 10.1 against 10.4 us, 2,150 items 13.9
+// against 12.1).
+constexpr int kTeam4MaxItems = 152 * 6;
+constexpr int team2_max_items(int dim) { return 152 * (dim >= 256 ? 12 : 16); }
+constexpr int plain_team_warps(int dim, int n_items) {
+  return n_items <= kTeam4MaxItems ? 4 : n_items <= team2_max_items(dim) ? 2 : 1;
+}
 constexpr int kMaxEdgeCap = 32;     // CSR entries per work item: one per lane
 
 }  // namespace de

@@ -83,6 +83,29 @@ __device__ __forceinline__ void force_lanes(const PlainBatchArgs &a, Frag<D> &ac
   if (k < cnt) force_group<D, U / 2, kAttract, kAfterWait>(a, acc, xi, ids, k, lr, bound, want_loss, loss, lane);
 }
 
+// Split rows: two-level, fixed-order combine of the parts; true on the warp that
+// ends up with the row's sum (every warp of an unsplit row).
+template <int D>
+__device__ __forceinline__ bool combine_parts(Frag<D> &acc, const WorkItem &it, float *slots, int32_t *counters,
+                                              int lane) {
+  if (it.nparts <= 1) return true;
+  const int P = it.nparts;
+  const int g = it.part / kCombineGroup;
+  const int ng = (P + kCombineGroup - 1) / kCombineGroup;
+  const int gsize = min(kCombineGroup, P - g * kCombineGroup);
+  store<D, true>(acc, slots + size_t(it.first_slot + it.part) * D, lane);
+  bool owner = arrive_last(counters + it.counter + g, gsize, lane);
+  if (owner) {
+    sum_slots(acc, slots + size_t(it.first_slot + g * kCombineGroup) * D, gsize, lane);
+    if (ng > 1) {
+      store<D, true>(acc, slots + size_t(it.first_slot + P + g) * D, lane);
+      owner = arrive_last(counters + it.counter + ng, ng, lane);
+      if (owner) sum_slots(acc, slots + size_t(it.first_slot + P) * D, ng, lane);
+    }
+  }
+  return owner;
+}
+
 // A row held in shared memory, in the Frag layout.
 template <int D>
 __device__ __forceinline__ void load_smem(Frag<D> &f, const float *row, int lane) {
@@ -218,24 +241,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
           force_lanes<D, U, false, true>(a, acc, xi, nid, kc, lr, bound, want_loss, loss, lane);
       }
 
-    // ---- split rows: two-level, fixed-order combine of the parts
-    bool owner = true;
-    if (it.nparts > 1) {
-      const int P = it.nparts;
-      const int g = it.part / kCombineGroup;
-      const int ng = (P + kCombineGroup - 1) / kCombineGroup;
-      const int gsize = min(kCombineGroup, P - g * kCombineGroup);
-      store<D, true>(acc, a.P + size_t(it.first_slot + it.part) * D, lane);
-      owner = arrive_last(a.counters + it.counter + g, gsize, lane);
-      if (owner) {
-        sum_slots(acc, a.P + size_t(it.first_slot + g * kCombineGroup) * D, gsize, lane);
-        if (ng > 1) {
-          store<D, true>(acc, a.P + size_t(it.first_slot + P + g) * D, lane);
-          owner = arrive_last(a.counters + it.counter + ng, ng, lane);
-          if (owner) sum_slots(acc, a.P + size_t(it.first_slot + P) * D, ng, lane);
-        }
-      }
-    }
+    const bool owner = combine_parts<D>(acc, it, a.P, a.counters, lane);
     // ---- update, staged (algo.hpp:651-666)
     if (owner) {
       Frag<D> out;
@@ -258,6 +264,118 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
     for (int m = 16; m >= 1; m >>= 1) loss += __shfl_xor_sync(kFull, loss, m);
     if (lane == 0) a.loss_partial[a.loss_off + gw] = double(loss);
   }
+}
+
+// ---------------------------------------------------------------- small minibatches
+//
+// The same step with W warps to a work item.  A minibatch that does not fill the
+// GPU takes as long as the longest chain in it, and a warp alone goes through a
+// row's groups of U pairs one after another (each a load, 17 shuffles and a divide:
+// about 0.6 us).  Here an item's CSR entries and then its draws are cut into groups
+// of U, group q on warp q % W, so a row of 32 entries and its draws is two rounds at
+// W = 4 instead of five; the warps' sums are added in warp order through shared
+// memory.  Phases, staging ring and split rows as in plain_batch_kernel.  Measured,
+// microseconds a minibatch, one warp an item -> this: 20,000-vertex kNN graph, dim
+// 128: B = 64 6.4 -> 3.4, 256 6.7 -> 4.0, 1024 8.3 -> 6.5; dim 256, B = 256 7.9 ->
+// 4.3; R-MAT of 100,003 vertices, dim 64, B = 512 6.3 -> 4.8.  Eight warps an item,
+// or groups of four pairs, gain at most 6 % below 100 items and lose above 300.
+template <int D, int U, int W>
+__global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBlocks)
+    plain_team_kernel(const PlainBatchArgs a) {
+  constexpr int kTeams = kPlainWarps / W;  // items of a CTA
+  constexpr int kRounds = 32 / U;          // groups of a warp whose ids its lanes hold at once
+  __shared__ float s_acc[kTeams][W - 1][D];
+  __shared__ float s_loss[kTeams][W - 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int team = warp / W, tw = warp % W;
+  const int item = blockIdx.x * kTeams + team;
+  const bool want_loss = a.compute_loss != 0;
+  const bool has_item = item < a.n_items;
+  WorkItem it{};
+  if (has_item) it = a.items[item];
+  const int epoch = a.epoch[0];
+  const float lr = a.lr[epoch], bound = a.bound;
+  const int skip = a.skip_last ? a.n - 1 : -1;  // edges into n-1 are dropped (algo.hpp:399-405, 538)
+  const int cnt = has_item ? it.e_end - it.e_begin : 0;
+  // the repulsive pass of a row is done by its part 0
+  const int rep_rows = (a.quirks && epoch + a.epoch[1] > 0) ? a.last_batch_size : a.rows;
+  const int32_t *negs = a.negs + (size_t(epoch) * a.batches + a.batch_id) * a.ns;
+  const int ge = (cnt + U - 1) / U;
+  const int groups = ge + (has_item && it.part == 0 && it.row < rep_rows ? (a.ns + U - 1) / U : 0);
+  // the other row of entry lane % U of this warp's group s + lane / U, -1 = none
+  auto fetch = [&](int s) -> int {
+    const int q = (s + lane / U) * W + tw, k = (q < ge ? q : q - ge) * U + lane % U;
+    int id = -1;
+    if (q < ge) {
+      if (k < cnt) id = __ldg(a.col + it.e_begin + k);
+      if (id == skip) id = -1;
+    } else if (q < groups) {
+      if (k < a.ns) id = __ldg(negs + k);
+      if (id >= a.n) id = -1;  // a draw equal to n contributes nothing
+    }
+    return id;
+  };
+  const int mine = groups > tw ? (groups - tw + W - 1) / W : 0;  // this warp's groups
+  float loss = 0.f;
+  Frag<D> xi, acc;
+  acc.zero();
+  int ids = mine > 0 ? fetch(0) : -1;
+  if (has_item) load_nc(xi, a.X + size_t(a.base + it.row) * D, lane);
+  // ---- before the wait: forces whose other row is final
+  for (int s = 0; s < mine; s += kRounds) {
+    if (s > 0) ids = fetch(s);
+    const int now = ids >= 0 && in_prev(a, ids) ? -1 : ids;
+    for (int r = 0; r < kRounds && s + r < mine; ++r) {
+      if ((s + r) * W + tw < ge)
+        force_group<D, U, true, false>(a, acc, xi, now, r * U, lr, bound, want_loss, loss, lane);
+      else
+        force_group<D, U, false, false>(a, acc, xi, now, r * U, lr, bound, want_loss, loss, lane);
+    }
+  }
+  pdl_wait();
+  pdl_trigger();
+  // ---- after the wait: forces into minibatch j-1
+  for (int s = 0; a.prev_rows > 0 && s < mine; s += kRounds) {
+    if (mine > kRounds) ids = fetch(s);
+    const int late = ids >= 0 && in_prev(a, ids) ? ids : -1;
+    if (!__any_sync(kFull, late >= 0)) continue;
+    for (int r = 0; r < kRounds && s + r < mine; ++r) {
+      if ((s + r) * W + tw < ge)
+        force_group<D, U, true, true>(a, acc, xi, late, r * U, lr, bound, want_loss, loss, lane);
+      else
+        force_group<D, U, false, true>(a, acc, xi, late, r * U, lr, bound, want_loss, loss, lane);
+    }
+  }
+  if (want_loss) {
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) loss += __shfl_xor_sync(kFull, loss, m);
+  }
+  // rows of minibatch j-1: staging buffer -> X, as in plain_batch_kernel
+  const int gw = blockIdx.x * kPlainWarps + warp, total_w = gridDim.x * kPlainWarps;
+  for (int r = gw; r < a.prev_rows; r += total_w) {
+    Frag<D> t;
+    load_cg(t, a.S_prev + size_t(r) * D, lane);
+    store<D, false>(t, a.X + size_t(a.prev_base + r) * D, lane);
+  }
+  if (tw > 0) {
+#pragma unroll
+    for (int t = 0; t < Frag<D>::N; ++t) s_acc[team][tw - 1][t * 32 + lane] = acc.v[t];
+    if (lane == 0) s_loss[team][tw - 1] = loss;
+  }
+  __syncthreads();
+  if (tw > 0 || !has_item) return;
+#pragma unroll
+  for (int w = 0; w < W - 1; ++w) {
+#pragma unroll
+    for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] += s_acc[team][w][t * 32 + lane];
+    loss += s_loss[team][w];
+  }
+  if (combine_parts<D>(acc, it, a.P, a.counters, lane)) {
+#pragma unroll
+    for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] = xi.v[t] + acc.v[t];
+    store<D, false>(acc, a.S_cur + size_t(it.row) * D, lane);
+  }
+  if (want_loss && lane == 0) a.loss_partial[a.loss_off + item] = double(loss);
 }
 
 // SpMMAlgo::algo_spmm's step at one rank (cpp/algo/spmm.hpp:54-159):
@@ -298,23 +416,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : (D == 128 ? 1
 #pragma unroll
       for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] = fmaf(a.lr, xn[u].v[t], acc.v[t]);
   }
-  bool owner = true;
-  if (it.nparts > 1) {
-    const int NP = it.nparts;
-    const int g = it.part / kCombineGroup;
-    const int ng = (NP + kCombineGroup - 1) / kCombineGroup;
-    const int gsize = min(kCombineGroup, NP - g * kCombineGroup);
-    store<D, true>(acc, P + size_t(it.first_slot + it.part) * D, lane);
-    owner = arrive_last(counters + it.counter + g, gsize, lane);
-    if (owner) {
-      sum_slots(acc, P + size_t(it.first_slot + g * kCombineGroup) * D, gsize, lane);
-      if (ng > 1) {
-        store<D, true>(acc, P + size_t(it.first_slot + NP + g) * D, lane);
-        owner = arrive_last(counters + it.counter + ng, ng, lane);
-        if (owner) sum_slots(acc, P + size_t(it.first_slot + NP) * D, ng, lane);
-      }
-    }
-  }
+  const bool owner = combine_parts<D>(acc, it, P, counters, lane);
   if (owner) store<D, false>(acc, a.Y + (size_t(j) * a.batch + it.row) * D, lane);
 }
 
@@ -397,10 +499,30 @@ cudaError_t launch(void (*k)(Args), int grid, int block, const Args &a, bool pdl
 
 }  // namespace
 
-cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, int grid, bool pdl, cudaStream_t s) {
+cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, bool teams, bool pdl, cudaStream_t s) {
   const int block = kPlainWarps * 32;
   if (a.stage_negs && a.ns > kStageNegMax) return cudaErrorInvalidValue;
   const size_t smem = a.stage_negs ? size_t(a.ns) * dim * sizeof(float) : 0;
+  const int w = teams ? plain_team_warps(dim, a.n_items) : 1;
+  const int grid = (a.n_items * w + kPlainWarps - 1) / kPlainWarps;
+  if (w == 4) {
+    switch (dim) {
+      case 32: return launch(plain_team_kernel<32, 8, 4>, grid, block, a, pdl, s);
+      case 64: return launch(plain_team_kernel<64, 8, 4>, grid, block, a, pdl, s);
+      case 128: return launch(plain_team_kernel<128, 8, 4>, grid, block, a, pdl, s);
+      case 256: return launch(plain_team_kernel<256, 4, 4>, grid, block, a, pdl, s);
+      default: return cudaErrorInvalidValue;
+    }
+  }
+  if (w == 2) {
+    switch (dim) {
+      case 32: return launch(plain_team_kernel<32, 8, 2>, grid, block, a, pdl, s);
+      case 64: return launch(plain_team_kernel<64, 8, 2>, grid, block, a, pdl, s);
+      case 128: return launch(plain_team_kernel<128, 8, 2>, grid, block, a, pdl, s);
+      case 256: return launch(plain_team_kernel<256, 4, 2>, grid, block, a, pdl, s);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   switch (dim) {
     case 32: return launch(plain_batch_kernel<32, 8>, grid, block, a, pdl, s, smem);
     case 64: return launch(plain_batch_kernel<64, 8>, grid, block, a, pdl, s, smem);

@@ -220,7 +220,6 @@ void build_schedule(const de_handle *h, int B, int cap, Schedule &s, std::vector
   s.item_off.assign(s.batches + 1, 0);
   s.n_parts.assign(s.batches, 0);
   s.n_split.assign(s.batches, 0);
-  s.cta_off.assign(s.batches + 1, 0);
   s.max_parts = s.max_split = 0;
   items.clear();
   for (int j = 0; j < s.batches; ++j) {
@@ -252,8 +251,6 @@ void build_schedule(const de_handle *h, int B, int cap, Schedule &s, std::vector
     s.n_split[j] = split;
     s.max_parts = std::max(s.max_parts, parts);
     s.max_split = std::max(s.max_split, split);
-    const int64_t n_items = s.item_off[j + 1] - s.item_off[j];
-    s.cta_off[j + 1] = s.cta_off[j] + (n_items + kPlainWarps - 1) / kPlainWarps;
   }
   s.n_items = int64_t(items.size());
 }
@@ -449,9 +446,9 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
     a.epoch = h->d_epoch;
     a.stage_negs = h->opt.stage_negatives && ns > 0 && ns <= kStageNegMax;
     a.err = h->d_err;
-    const int grid = int(s.cta_off[j + 1] - s.cta_off[j]);
     if (ev) cudaEventRecord(ev[j], st);
-    err = launch_plain_batch(h->dim, a, grid, h->opt.pdl && j > 0 && !ev, st);
+    // a caller that sets the edge cap asks for one warp a work item of that size
+    err = launch_plain_batch(h->dim, a, h->opt.edge_cap <= 0 && !a.stage_negs, h->opt.pdl && j > 0 && !ev, st);
   }
   if (err == cudaSuccess) {
     FlushArgs f{};
