@@ -89,6 +89,7 @@ struct PlainBatchArgs {
   int32_t prev_base, prev_rows;    // minibatch j-1 (prev_rows = 0: none)
   int32_t prev2_base, prev2_rows;  // minibatch j-2 (prev2_rows = 0: none)
   int32_t batch_id, batches, last_batch_size;
+  int32_t first;            // 1: launched with a programmatic dependency, but nothing may be read before its end
   int32_t n;
   int32_t quirks, compute_loss;
   int32_t skip_last;        // F7: edges into vertex n-1 are dropped
@@ -122,6 +123,7 @@ struct FlushArgs {
 };
 
 constexpr int kFlushBlocks = 152;
+constexpr int64_t kFlushChunk = 2048;  // loss partials of a CTA at least: eight a thread, one round of loads
 
 // The SpMM step (spmm_kernel): every work item of every minibatch in one launch,
 // y rows from the unchanged input x; a minibatch's split rows use partial slots

@@ -156,6 +156,8 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
   const int total_w = gridDim.x * kPlainWarps;
   const bool want_loss = a.compute_loss != 0;
 
+  // an epoch's first minibatch reads what the launch before it writes
+  if (a.first) pdl_wait();
   const bool has_item = gw < a.n_items;
   WorkItem it{};
   if (has_item) it = a.items[gw];
@@ -290,6 +292,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
   const int team = warp / W, tw = warp % W;
   const int item = blockIdx.x * kTeams + team;
   const bool want_loss = a.compute_loss != 0;
+  if (a.first) pdl_wait();  // as in plain_batch_kernel
   const bool has_item = item < a.n_items;
   WorkItem it{};
   if (has_item) it = a.items[item];
@@ -420,6 +423,29 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : (D == 128 ? 1
   if (owner) store<D, false>(acc, a.Y + (size_t(j) * a.batch + it.row) * D, lane);
 }
 
+// v[0] + ... + v[n - 1] by a CTA of 256 threads in a fixed order; on thread 0.
+__device__ __forceinline__ double block_sum(const double *v, int64_t n, double *red) {
+  double s = 0.0;
+  int64_t i = threadIdx.x;
+  for (; i + 7 * 256 < n; i += 8 * 256) {  // eight loads in flight, added in order
+    double t[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) t[u] = __ldcg(v + i + u * 256);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += t[u];
+  }
+  for (; i < n; i += 256) s += __ldcg(v + i);
+#pragma unroll
+  for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(kFull, s, m);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < 8; ++w) s += red[w];
+  return s;
+}
+
 // End of an epoch: write back the last minibatch, reduce the epoch's loss
 // partials in a fixed order (each CTA a fixed chunk, then the last CTA to
 // finish sums the chunk sums in order), advance the epoch counter.
@@ -429,44 +455,41 @@ __global__ void __launch_bounds__(256) flush_kernel(const FlushArgs a) {
   const int gw = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int total_w = gridDim.x * 8;
   pdl_wait();
+  pdl_trigger();
   for (int r = gw; r < a.last_rows; r += total_w) {
     Frag<D> t;
     load_nc(t, a.S_last + size_t(r) * D, lane);
     store<D, false>(t, a.X + size_t(a.last_base + r) * D, lane);
   }
-  __shared__ double red[256];
+  if (!a.compute_loss) {
+    // every reader of the epoch counter was in the launches before this one
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.epoch[0] += 1;
+    return;
+  }
+  // The loss: kFlushChunk partials a CTA (or more, where the grid is too small), so
+  // a small job's sum needs no second step across CTAs.
+  const int64_t per = (a.n_partials + gridDim.x - 1) / gridDim.x;
+  const int64_t chunk = per > kFlushChunk ? per : kFlushChunk;
+  const int parts = int((a.n_partials + chunk - 1) / chunk);
+  if (int(blockIdx.x) >= parts) return;
+  __shared__ double red[8];
   __shared__ bool last;
-  double s = 0.0;
-  if (a.compute_loss) {
-    const int64_t chunk = (a.n_partials + gridDim.x - 1) / gridDim.x;
-    const int64_t lo = blockIdx.x * chunk, hi = min(a.n_partials, lo + chunk);
-    for (int64_t i = lo + threadIdx.x; i < hi; i += 256) s += a.loss_partial[i];
-  }
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+  const int64_t lo = blockIdx.x * chunk;
+  double s = block_sum(a.loss_partial + lo, min(a.n_partials - lo, chunk), red);
+  if (parts > 1) {
+    if (threadIdx.x == 0) {
+      a.block_sums[blockIdx.x] = s;
+      __threadfence();
+      last = atomicAdd(a.done, 1) == parts - 1;
+    }
     __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    a.block_sums[blockIdx.x] = red[0];
+    if (!last) return;
     __threadfence();
-    last = atomicAdd(a.done, 1) == int(gridDim.x) - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  s = 0.0;
-  for (int b = threadIdx.x; b < int(gridDim.x); b += 256) s += __ldcg(a.block_sums + b);
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+    s = block_sum(a.block_sums, parts, red);
   }
   if (threadIdx.x == 0) {
     const int e = a.epoch[0];
-    if (a.compute_loss) a.loss[e] = red[0];
+    a.loss[e] = s;
     a.epoch[0] = e + 1;
     *a.done = 0;
   }

@@ -429,6 +429,7 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
     a.prev2_base = j > 1 ? int32_t(int64_t(j - 2) * s.batch) : 0;
     a.prev2_rows = j > 1 ? s.batch : 0;
     a.batch_id = j;
+    a.first = j == 0;
     a.batches = s.batches;
     a.last_batch_size = s.last_batch_size;
     a.n = int32_t(h->n);
@@ -448,7 +449,7 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
     a.err = h->d_err;
     if (ev) cudaEventRecord(ev[j], st);
     // a caller that sets the edge cap asks for one warp a work item of that size
-    err = launch_plain_batch(h->dim, a, h->opt.edge_cap <= 0 && !a.stage_negs, h->opt.pdl && j > 0 && !ev, st);
+    err = launch_plain_batch(h->dim, a, h->opt.edge_cap <= 0 && !a.stage_negs, h->opt.pdl && !ev, st);
   }
   if (err == cudaSuccess) {
     FlushArgs f{};
@@ -485,6 +486,13 @@ cudaError_t enqueue_epoch(de_handle *h, int ns, cudaStream_t st, cudaEvent_t *ev
   return h->opt.precision == DE_PRECISION_BF16 ? enqueue_epoch_bf16(h, ns, st, ev)
                                                : enqueue_epoch_plain(h, ns, st, ev);
 }
+
+// Epochs of at most this many minibatches are launched kernel by kernel: a graph
+// launch per epoch costs more than two to five launches that overlap, and its
+// capture falls away from the first run.  Measured, 10 to 20 epochs, dim 32, us a
+// run by graph -> by launches: 1 minibatch 272 -> 210 (first run 466 -> 395),
+// 3 441 -> 437 (1335 -> 1293), 8 642 -> 647, 34 1351 -> 1442.
+constexpr int kDirectBatches = 4;
 
 int capture_epoch(de_handle *h, int ns) {
   const Schedule &s = h->sched;
@@ -849,11 +857,15 @@ int de_run_from(de_handle *h, int32_t first_epoch, int32_t epochs, int32_t batch
   int rc = prepare_run(h, first_epoch, epochs, batch_size, ns, lr_per_epoch);
   if (rc) return rc;
   const Schedule &s = h->sched;
-  if (!h->graph || h->graph_batch != s.batch || h->graph_ns != ns) {
-    drop_graph(h);
-    if ((rc = capture_epoch(h, ns))) return rc;
+  if (h->opt.precision == DE_PRECISION_FP32 && s.batches <= kDirectBatches) {
+    for (int i = 0; i < epochs; ++i) DE_CUDA(h, enqueue_epoch(h, ns, h->stream, nullptr));
+  } else {
+    if (!h->graph || h->graph_batch != s.batch || h->graph_ns != ns) {
+      drop_graph(h);
+      if ((rc = capture_epoch(h, ns))) return rc;
+    }
+    for (int i = 0; i < epochs; ++i) DE_CUDA(h, cudaGraphLaunch(h->graph, h->stream));
   }
-  for (int i = 0; i < epochs; ++i) DE_CUDA(h, cudaGraphLaunch(h->graph, h->stream));
   if (loss_per_epoch) {
     DE_CUDA(h, cudaMemcpyAsync(h->h_loss, h->d_loss, epochs * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     DE_CUDA(h, cudaStreamSynchronize(h->stream));
