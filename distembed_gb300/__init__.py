@@ -198,7 +198,9 @@ def _take_csr(L, rc, h):
         L.de_csr_info(h, ctypes.byref(r), ctypes.byref(c), ctypes.byref(z))
         rowptr = np.zeros(r.value + 1, dtype=np.int64)
         col = np.zeros(max(z.value, 1), dtype=np.int64)
-        L.de_csr_copy(h, rowptr.ctypes.data, col.ctypes.data)
+        rc = L.de_csr_copy(h, rowptr.ctypes.data, col.ctypes.data)
+        if rc != DE_OK:
+            raise DEError(rc, L.de_last_error(None).decode())
         return r.value, c.value, rowptr, col[: z.value]
     finally:
         L.de_csr_free(h)

@@ -213,8 +213,12 @@ int main(int argc, char **argv) {
     de_csr_info(c, &rows, &cols, &nnz);
     csr.rowStart.resize(size_t(rows) + 1);
     csr.col_idx.resize(size_t(nnz > 0 ? nnz : 1));
-    de_csr_copy(c, csr.rowStart.data(), csr.col_idx.data());
+    const int rc = de_csr_copy(c, csr.rowStart.data(), csr.col_idx.data());
     de_csr_free(c);
+    if (rc != DE_OK) {
+      std::fprintf(stderr, "reading %s: %s\n", f.input.c_str(), de_last_error(nullptr));
+      return 1;
+    }
   } else {
     if (de_mm_read(f.input.c_str(), &rows, &cols, &nnz, nullptr, nullptr, 0) != DE_OK) {
       std::fprintf(stderr, "reading %s: %s\n", f.input.c_str(), de_last_error(nullptr));

@@ -334,7 +334,8 @@ int de_mm_read_gpu(const char *path, int32_t device, de_csr **out);
 int de_coo_to_csr(int64_t rows, int64_t cols, const int64_t *row_idx, const int64_t *col_idx, int64_t nnz,
                   int32_t mirror, int32_t device, de_csr **out);
 int de_csr_info(const de_csr *c, int64_t *rows, int64_t *cols, int64_t *nnz);
-/* rowptr[rows + 1], col[nnz]. */
+/* Copies the CSR, which stays on the GPU until de_csr_free, to host arrays
+ * rowptr[rows + 1] and col[nnz]. */
 int de_csr_copy(const de_csr *c, int64_t *rowptr, int64_t *col);
 void de_csr_free(de_csr *c);
 /* Embedding writer of ParallelIO::parallel_write (cpp/io/parrallel_IO.hpp:90-146):
