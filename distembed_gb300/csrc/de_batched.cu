@@ -1,9 +1,10 @@
 // Batched form: many independent graphs in one persistent launch (sm_103a).
 //
-// Each graph is owned by one CTA (a "team") for all its epochs, so the
-// reference's minibatch order (cpp/algo/algo.hpp:164-192: batch b+1 reads the
-// update of batch b, rows of one batch read pre-batch values) needs nothing but
-// __syncthreads: no grid-wide barrier and no waiting on other CTAs.  Teams take
+// Each graph is owned by one CTA or one cluster of CTAs (a "team") for all its
+// epochs, so the reference's minibatch order (cpp/algo/algo.hpp:164-192: batch b+1
+// reads the update of batch b, rows of one batch read pre-batch values) needs
+// nothing but __syncthreads or the cluster's hardware barrier: no grid-wide barrier
+// and no waiting on CTAs that may not be running.  Teams take
 // graphs largest first from an atomic counter.  Per minibatch:
 //   1. work items (a row, or a <= cap-edge piece of a high-degree row) are spread
 //      over the team's warps; a warp runs VPW items at once, each on 32/VPW lanes;
@@ -17,8 +18,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
+#include <queue>
 #include <random>
 #include <string>
 #include <vector>
@@ -131,6 +135,7 @@ struct de_batch {
   // per (batch size, edge cap) schedule
   int sched_batch = 0, sched_cap = 0;
   std::vector<GraphInfo> ginfo;
+  std::vector<int64_t> graph_items;  // work items of each graph
   std::vector<int32_t> order;
   GraphInfo *d_graphs = nullptr;
   int32_t *d_order = nullptr, *d_next = nullptr;
@@ -199,6 +204,7 @@ int build_batched_schedule(de_batch *b, int B, int cap) {
   std::vector<int32_t> bsplit{0};
   std::vector<SplitRow> splits;
   b->ginfo.assign(b->n_graphs, GraphInfo{});
+  b->graph_items.assign(b->n_graphs, 0);
   int max_slots = 1;
   int64_t max_items = 1;
   int64_t batch_off = 0;
@@ -240,6 +246,7 @@ int build_batched_schedule(de_batch *b, int B, int cap) {
       bsplit.push_back(int32_t(splits.size()));
     }
     batch_off += G.batches;
+    b->graph_items[g] = bitem.back() - bitem[size_t(G.batch_off)];
   }
   b->sched_batch = B;
   b->sched_cap = cap;
@@ -274,11 +281,47 @@ int build_batched_schedule(de_batch *b, int B, int cap) {
   return DE_OK;
 }
 
-int teams_for(de_batch *b, const KernelPick &k) {
+// CTAs to a team of the register kernel: 1, 2, 4 or 8 (a portable cluster), whichever
+// ends first when the graphs go largest first to the teams that fit the GPU at once.
+// A minibatch costs a team its barriers and update and, per round of its warps over
+// the minibatch's items, the chain of loads of the longest row; the two constants
+// only have to rank the sizes (256 rows a minibatch, vertices_per_warp 4, 8 warps:
+// about 57 us at one CTA, 8 rounds, 10 us at eight).  Measured, ms for two epochs at
+// 1 / 2 / 4 / 8 CTAs a team: 24 graphs of 500-5,000, dim 32: 2.03 / 1.23 / 0.79 /
+// 0.58; 64 of 500-50,000, dim 64: 30.1 / 17.3 / 12.3 / 8.6; 256 of 500-10,000, dim
+// 64: 6.5 / 4.2 / 3.0 / 4.3; dim 32, 512 rows: 4.7 / 2.6 / 3.1 / 4.9.  The rule took
+// the smallest of each.
+int register_ctas(const de_batch *b, const de_batch_shape &s, int resident) {
+  constexpr double kFixedUs = 4.0, kRoundUs = 6.5;
+  int best = 1;
+  double best_us = -1;
+  for (int ctas : {1, 2, 4, 8}) {
+    const int per_round = ctas * s.team_warps * s.vertices_per_warp;
+    const int teams = std::min(resident / ctas, b->n_graphs);
+    if (teams < 1) break;
+    std::priority_queue<double, std::vector<double>, std::greater<double>> busy;  // when each team is free
+    for (int t = 0; t < teams; ++t) busy.push(0.0);
+    double end = 0;
+    for (int g : b->order) {
+      const GraphInfo &G = b->ginfo[g];
+      const double items = double(b->graph_items[g]) / G.batches;
+      const double us = busy.top() + G.batches * (kFixedUs + kRoundUs * std::ceil(items / per_round));
+      busy.pop();
+      busy.push(us);
+      end = std::max(end, us);
+    }
+    if (best_us < 0 || end < best_us) best = ctas, best_us = end;
+  }
+  return best;
+}
+
+int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape) {
   int per_sm = 0, sms = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.block, k.smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || sms < 1) sms = 1;
+  const bool reg = shape.kernel == DE_BATCH_REGISTER;
+  if (reg) k.ctas = register_ctas(b, shape, per_sm * sms);
   if (k.ctas == 1) return std::min(per_sm * sms, b->n_graphs);
   // clusters of k.ctas CTAs: as many as can be resident at once (a cluster sits in one GPC)
   cudaLaunchConfig_t cfg{};
@@ -297,7 +340,9 @@ int teams_for(de_batch *b, const KernelPick &k) {
     cudaGetLastError();
     clusters = std::max(1, per_sm * sms / k.ctas);
   }
-  return k.ctas * std::min(clusters, (b->n_graphs + k.ctas - 1) / k.ctas);
+  // a register team of several CTAs takes one graph; the CTAs of a staged one take
+  // the smaller graphs alone
+  return k.ctas * std::min(clusters, reg ? b->n_graphs : (b->n_graphs + k.ctas - 1) / k.ctas);
 }
 
 // Everything of a run except the launch: schedule, negatives, rates, team staging
@@ -307,7 +352,7 @@ int prepare_batched(de_batch *b, int epochs, int B, int ns, const double *lr, co
   BCUDA(b, cudaSetDevice(b->device));
   if (shape.kernel != DE_BATCH_REGISTER && ns > kStagedMaxNs)
     return bfail(b, DE_ERR_UNSUPPORTED, "the staged kernel takes at most 32 negatives per minibatch");
-  const KernelPick k = pick_kernel(b->dim, b->opt.precision == DE_PRECISION_BF16, shape, ns);
+  KernelPick k = pick_kernel(b->dim, b->opt.precision == DE_PRECISION_BF16, shape, ns);
   if (!k.fn) return bfail(b, DE_ERR_UNSUPPORTED, "no kernel for this dim and team shape (or its shared memory is too large)");
   if (k.smem) BCUDA(b, cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.smem)));
   const int cap = shape.edge_cap;
@@ -346,31 +391,29 @@ int prepare_batched(de_batch *b, int epochs, int B, int ns, const double *lr, co
   BCUDA(b, cudaMemcpyAsync(b->d_lr, lrf.data(), epochs * sizeof(float), cudaMemcpyHostToDevice, b->stream));
   BCUDA(b, cudaMemcpyAsync(b->d_graphs, b->ginfo.data(), b->ginfo.size() * sizeof(GraphInfo), cudaMemcpyHostToDevice,
                            b->stream));
-  BCUDA(b, cudaStreamSynchronize(b->stream));
-  const int teams = teams_for(b, k);
+  // graphs largest first by work (CSR entries, repulsive pairs and a fixed cost per
+  // minibatch, all per epoch)
+  std::vector<double> w(b->n_graphs);
+  double total_w = 0;
+  for (int g = 0; g < b->n_graphs; ++g) {
+    w[g] = double(b->nnz[g]) + double(ns) * double(b->n[g]) + 900.0 * b->ginfo[g].batches;
+    total_w += w[g];
+  }
+  std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) { return w[x] > w[y]; });
+  const int teams = teams_for(b, k, shape);
+  // with staged teams of several CTAs the graphs above 0.6 of the balanced share of
+  // one CTA are trained by a whole cluster
+  b->n_big = 0;
+  if (k.ctas > 1 && shape.kernel != DE_BATCH_REGISTER)
+    while (b->n_big < b->n_graphs && w[b->order[b->n_big]] > 0.6 * total_w / teams) ++b->n_big;
+  BCUDA(b, cudaMemcpyAsync(b->d_order, b->order.data(), b->order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
+                           b->stream));
+  BCUDA(b, cudaStreamSynchronize(b->stream));  // the host vectors go away on return
   if (int rc = bgrow(b, &b->d_stage, &b->stage_cap, size_t(teams) * B * b->dim)) return rc;
   if (int rc = bgrow(b, &b->d_slots, &b->slots_cap, size_t(teams) * b->max_slots * b->dim)) return rc;
   if (int rc = bgrow(b, &b->d_item_loss, &b->item_loss_cap, size_t(teams) * b->max_batch_items)) return rc;
   if (int rc = bgrow(b, &b->d_cluster_slot, &b->cluster_slot_cap, size_t(teams / std::max(k.ctas, 1) + 1)))
     return rc;
-  // graphs largest first by work (CSR entries, repulsive pairs and a fixed cost per
-  // minibatch, all per epoch); with two-CTA teams the graphs above 0.6 of the
-  // balanced share of one CTA are trained by a whole cluster
-  {
-    std::vector<double> w(b->n_graphs);
-    double total_w = 0;
-    for (int g = 0; g < b->n_graphs; ++g) {
-      w[g] = double(b->nnz[g]) + double(ns) * double(b->n[g]) + 900.0 * b->ginfo[g].batches;
-      total_w += w[g];
-    }
-    std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) { return w[x] > w[y]; });
-    b->n_big = 0;
-    if (k.ctas > 1)
-      while (b->n_big < b->n_graphs && w[b->order[b->n_big]] > 0.6 * total_w / teams) ++b->n_big;
-    BCUDA(b, cudaMemcpyAsync(b->d_order, b->order.data(), b->order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
-                             b->stream));
-    BCUDA(b, cudaStreamSynchronize(b->stream));
-  }
   BatchedArgs &a = b->args;
   a = BatchedArgs{};
   a.graphs = b->d_graphs;

@@ -60,7 +60,7 @@ struct BatchedArgs {
   // single CTAs (next_graph counts from order[n_big])
   int32_t n_big;
   int32_t *next_big;
-  int32_t *cluster_slot;     // [clusters] graph handed from CTA rank 0 to rank 1
+  int32_t *cluster_slot;     // [clusters] graph handed from CTA rank 0 to the others
   float *item_loss;          // [teams, max items of a minibatch] loss of every work item
   int32_t item_stride;
   int32_t loss_from;         // epochs e >= loss_from (of this run) compute their loss; the others write 0
@@ -71,6 +71,34 @@ static __device__ __forceinline__ long long globaltimer() {
   long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
+}
+
+static __device__ __forceinline__ int cluster_rank() {
+  int r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+// CTAs of this CTA's cluster (1 without a cluster launch).
+static __device__ __forceinline__ int cluster_ctas() {
+  int r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+
+// Every CTA of the cluster: every thread arrives (release) and waits (acquire),
+// so each CTA's global writes before the barrier are visible to the others after it.
+static __device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A minibatch's loss from its items' losses, in item order (one warp).
+static __device__ __forceinline__ double minibatch_loss(const float *item_loss, int n_items, int lane) {
+  double l = 0.0;
+  for (int i = lane; i < n_items; i += 32) l += double(__ldcg(item_loss + i));
+#pragma unroll
+  for (int m = 16; m >= 1; m >>= 1) l += __shfl_xor_sync(kAll, l, m);
+  return l;
 }
 
 static __device__ __forceinline__ float bclip(float v, float b) { return v > b ? b : (v < -b ? -b : v); }

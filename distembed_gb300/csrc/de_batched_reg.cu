@@ -1,5 +1,7 @@
 // Batched form, register kernel: a warp runs vertices_per_warp work items at once
-// on 32 / vertices_per_warp lanes each, neighbour rows loaded into registers.
+// on 32 / vertices_per_warp lanes each, neighbour rows loaded into registers.  A
+// team is one CTA, or the CTAs of a cluster where the graphs alone would leave SMs
+// idle (register_ctas in de_batched.cu); a graph's results do not depend on which.
 #include "de_batched.cuh"
 
 namespace de {
@@ -19,21 +21,41 @@ template <int D, int VPW, bool kBF16>
 __device__ __forceinline__ void load_row(Row<D, VPW> &r, const BatchedArgs &a, int64_t vertex, int gl) {
   constexpr int P = Row<D, VPW>::P;
   const int64_t base = vertex * D + int64_t(gl) * P;
+  // widest loads the lane's P components allow (rows and lane offsets are P-aligned)
   if constexpr (kBF16) {
-    const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162 *>(a.xb + base);
+    constexpr int K = P % 8 == 0 ? 4 : P % 4 == 0 ? 2 : 1;  // 32-bit words per load
+    const uint32_t *p = reinterpret_cast<const uint32_t *>(a.xb + base);
 #pragma unroll
-    for (int i = 0; i < P / 2; ++i) {
-      float2 f = __bfloat1622float2(p[i]);
-      r.v[2 * i] = f.x;
-      r.v[2 * i + 1] = f.y;
+    for (int i = 0; i < P / 2; i += K) {
+      uint32_t w[K];
+      if constexpr (K == 4) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(p + i);
+        w[0] = u.x, w[1] = u.y, w[2] = u.z, w[3] = u.w;
+      } else if constexpr (K == 2) {
+        const uint2 u = *reinterpret_cast<const uint2 *>(p + i);
+        w[0] = u.x, w[1] = u.y;
+      } else {
+        w[0] = p[i];
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        r.v[2 * (i + k)] = __uint_as_float(w[k] << 16);
+        r.v[2 * (i + k) + 1] = __uint_as_float(w[k] & 0xffff0000u);
+      }
+    }
+  } else if constexpr (P % 4 == 0) {
+    const float4 *p = reinterpret_cast<const float4 *>(a.xm + base);
+#pragma unroll
+    for (int i = 0; i < P / 4; ++i) {
+      const float4 f = __ldcg(p + i);
+      r.v[4 * i] = f.x, r.v[4 * i + 1] = f.y, r.v[4 * i + 2] = f.z, r.v[4 * i + 3] = f.w;
     }
   } else {
     const float2 *p = reinterpret_cast<const float2 *>(a.xm + base);
 #pragma unroll
     for (int i = 0; i < P / 2; ++i) {
-      float2 f = __ldcg(p + i);
-      r.v[2 * i] = f.x;
-      r.v[2 * i + 1] = f.y;
+      const float2 f = __ldcg(p + i);
+      r.v[2 * i] = f.x, r.v[2 * i + 1] = f.y;
     }
   }
 }
@@ -45,7 +67,11 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 
-// Forces of up to 4 rows named by lanes [k, k+4) of the group (ids < 0: none),
+// Rows in flight per group: eight where a lane's share of a row is small.
+template <int D, int VPW>
+constexpr int kInFlight = Row<D, VPW>::L >= 8 && Row<D, VPW>::P <= 4 ? 8 : 4;
+
+// Forces of up to kInFlight rows named by lanes [k, k + kInFlight) of the group (ids < 0: none),
 // all groups of the warp in step (the caller keeps the warp converged).  xi is the
 // row's FP32 master value.  In the BF16 form the rows are read as BF16; a pair
 // whose squared distance from those reads is below a.near_r is read again from
@@ -56,7 +82,7 @@ __device__ __forceinline__ void group_forces(const BatchedArgs &a, Row<D, VPW> &
                                              int64_t voff, int ids, int k, int gbase, int gl, float lr,
                                              float &loss, bool want) {
   constexpr int L = Row<D, VPW>::L, P = Row<D, VPW>::P;
-  constexpr int U = L >= 4 ? 4 : L;
+  constexpr int U = kInFlight<D, VPW>;
   Row<D, VPW> xn[U];
   int nid[U];
   float r[U];
@@ -113,26 +139,36 @@ __device__ __forceinline__ void group_forces(const BatchedArgs &a, Row<D, VPW> &
 
 template <int D, int VPW, int WARPS, bool kBF16>
 __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a) {
-  constexpr int L = Row<D, VPW>::L, P = Row<D, VPW>::P;
+  constexpr int L = Row<D, VPW>::L, P = Row<D, VPW>::P, U = kInFlight<D, VPW>;
   static_assert(P % 2 == 0, "components per lane must be even");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane / L, gl = lane % L, gbase = grp * L;
   __shared__ int sh_graph;
-  __shared__ double sh_loss[WARPS];
-  float *stage = a.stage + size_t(blockIdx.x) * a.batch * D;
-  float *slots = a.slots + size_t(blockIdx.x) * a.slot_stride * D;
+  // team: nct CTAs (those of the cluster), this one its rank-th
+  const int nct = cluster_ctas(), rank = nct > 1 ? cluster_rank() : 0;
+  const int team = blockIdx.x / nct, tw = rank * WARPS + warp, TW = nct * WARPS;
+  auto team_sync = [&]() {
+    if (nct > 1) cluster_sync();
+    else __syncthreads();
+  };
+  float *stage = a.stage + size_t(team) * a.batch * D;
+  float *slots = a.slots + size_t(team) * a.slot_stride * D;
+  float *item_loss = a.item_loss + size_t(team) * a.item_stride;
   const int skip_last = a.quirks;
 
   for (;;) {
-    if (threadIdx.x == 0) {
+    int g;
+    if (threadIdx.x == 0 && rank == 0) {
       const int i = atomicAdd(a.next_graph, 1);
-      sh_graph = i < a.n_graphs ? a.order[i] : -1;
+      g = i < a.n_graphs ? a.order[i] : -1;
+      if (nct > 1) *reinterpret_cast<volatile int *>(a.cluster_slot + team) = g;
+      else sh_graph = g;
     }
-    __syncthreads();
-    const int g = sh_graph;
-    __syncthreads();
+    team_sync();
+    g = nct > 1 ? __ldcg(a.cluster_slot + team) : sh_graph;
+    team_sync();  // the slot is rewritten only after every thread has read it
     if (g < 0) return;
-    if (a.trace && threadIdx.x == 0) {
+    if (a.trace && threadIdx.x == 0 && rank == 0) {
       a.trace[3 * g] = globaltimer();
       a.trace[3 * g + 2] = blockIdx.x;
     }
@@ -141,7 +177,7 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
     for (int e = 0; e < a.epochs; ++e) {
       const float lr = a.lr[e];
       const bool want = a.compute_loss && e >= a.loss_from;
-      double wloss = 0.0;  // this warp's share of the epoch loss, in item order
+      double eloss = 0.0;  // rank 0, warp 0: the epoch's loss, minibatch by minibatch
       for (int j = 0; j < G.batches; ++j) {
         const int64_t bi = G.batch_off + j;
         const int64_t it0 = a.batch_item_off[bi];
@@ -151,7 +187,7 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
         const int rep_rows = (a.quirks && e > 0) ? G.last_batch_size : rows;  // algo.hpp:167-169, 594
         const int32_t *negs = a.negs + G.neg_off + (size_t(e) * G.batches + j) * a.ns;
         // ---- 1. items, VPW per warp at a time
-        for (int i0 = warp * VPW; i0 < n_items; i0 += WARPS * VPW) {
+        for (int i0 = tw * VPW; i0 < n_items; i0 += TW * VPW) {
           const int my = i0 + grp;
           const bool has = my < n_items;
           WorkItem it{};
@@ -165,16 +201,15 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
             for (int t = 0; t < P; ++t) xi.v[t] = 0.f;
           float loss = 0.f;
           const int cnt = has ? it.e_end - it.e_begin : 0;
+          const int32_t *cols = a.col + G.eoff + it.e_begin;
           int maxcnt = cnt;
 #pragma unroll
           for (int m = 16; m >= L; m >>= 1) maxcnt = max(maxcnt, __shfl_xor_sync(kAll, maxcnt, m));
+          int next = gl < cnt ? __ldg(cols + gl) : -1;
           for (int c0 = 0; c0 < maxcnt; c0 += L) {
-            int ids = -1;
-            if (gl < cnt - c0) {
-              ids = __ldg(a.col + G.eoff + it.e_begin + c0 + gl);
-              if (ids == skip) ids = -1;
-            }
-            for (int k = 0; k < L && c0 + k < maxcnt; k += (L >= 4 ? 4 : L))
+            const int ids = next == skip ? -1 : next;
+            next = gl < cnt - c0 - L ? __ldg(cols + c0 + L + gl) : -1;  // the next chunk's ids, a chunk ahead
+            for (int k = 0; k < L && c0 + k < maxcnt; k += U)
               group_forces<D, VPW, kBF16, true>(a, acc, xi, G.voff, ids, k, gbase, gl, lr, loss, want);
           }
           const bool repulse = has && it.part == 0 && it.row < rep_rows;
@@ -185,36 +220,31 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
               ids = __ldg(negs + k0 + gl);
               if (ids >= G.n) ids = -1;  // a draw equal to n contributes nothing
             }
-            for (int k = 0; k < L && k0 + k < a.ns; k += (L >= 4 ? 4 : L))
+            for (int k = 0; k < L && k0 + k < a.ns; k += U)
               group_forces<D, VPW, kBF16, false>(a, acc, xi, G.voff, ids, k, gbase, gl, lr, loss, want);
           }
           if (has) {
             float *dst = it.nparts > 1 ? slots + size_t(it.first_slot + it.part) * D : stage + size_t(it.row) * D;
 #pragma unroll
             for (int t = 0; t < P; t += 2) *reinterpret_cast<float2 *>(dst + gl * P + t) = make_float2(acc.v[t], acc.v[t + 1]);
+            if (want && gl == 0) item_loss[my] = loss;
           }
-          // item loss, fixed order: groups of the warp in order
-#pragma unroll
-          for (int q = 0; q < VPW; ++q) wloss += double(__shfl_sync(kAll, loss, q * L));
         }
-        __syncthreads();
+        team_sync();
         // ---- 2. split rows: pieces in piece order
-        combine_split_rows<D>(a, slots, stage, a.batch_split_off[bi], a.batch_split_off[bi + 1], warp, WARPS, lane);
-        __syncthreads();
+        const int s0 = a.batch_split_off[bi], s1 = a.batch_split_off[bi + 1];
+        combine_split_rows<D>(a, slots, stage, s0, s1, tw, TW, lane);
+        // the minibatch's loss in item order, whatever team made it
+        if (want && tw == 0) eloss += minibatch_loss(item_loss, n_items, lane);
+        if (s1 > s0) team_sync();
         // ---- 3. update (algo.hpp:651-666)
-        update_rows<kBF16>(a.xm, a.xb, stage, (G.voff + base) * D, rows * D, threadIdx.x, WARPS * 32);
-        __syncthreads();
+        update_rows<kBF16>(a.xm, a.xb, stage, (G.voff + base) * D, rows * D, rank * WARPS * 32 + threadIdx.x,
+                           TW * 32);
+        team_sync();
       }
-      if (lane == 0) sh_loss[warp] = wloss;
-      __syncthreads();
-      if (threadIdx.x == 0 && a.compute_loss) {
-        double s = 0.0;
-        for (int w = 0; w < WARPS; ++w) s += sh_loss[w];
-        a.loss[size_t(g) * a.epochs + e] = s;
-      }
-      __syncthreads();
+      if (tw == 0 && lane == 0 && a.compute_loss) a.loss[size_t(g) * a.epochs + e] = eloss;
     }
-    if (a.trace && threadIdx.x == 0) a.trace[3 * g + 1] = globaltimer();
+    if (a.trace && threadIdx.x == 0 && rank == 0) a.trace[3 * g + 1] = globaltimer();
   }
 }
 

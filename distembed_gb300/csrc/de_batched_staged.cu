@@ -133,18 +133,6 @@ __device__ __forceinline__ void staged_pairs(const BatchedArgs &a, float (&acc)[
 }
 
 
-__device__ __forceinline__ int cluster_rank() {
-  int r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-// Every CTA of the cluster: every thread arrives (release) and waits (acquire),
-// so each CTA's global writes before the barrier are visible to the others after it.
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // A team is one CTA or, with CT = 2 or 4, the CTAs of a cluster working on one
 // graph: team warp tw = rank * W + warp of TW = nct * W, one shared staging area
 // (that of rank 0), barriers across the cluster.  With CT > 1 a cluster first
@@ -329,13 +317,7 @@ __global__ void __launch_bounds__(512, 1) staged_kernel(const BatchedArgs a) {
         const int s0 = a.batch_split_off[bi], s1 = a.batch_split_off[bi + 1];
         combine_split_rows<D>(a, slots, stage, s0, s1, tw, TW, lane);
         // the minibatch's loss in item order (rank 0, warp 0), whatever team made it
-        if (want && trank == 0 && warp == 0) {
-          double l = 0.0;
-          for (int i = lane; i < n_items; i += 32) l += double(__ldcg(item_loss + i));
-#pragma unroll
-          for (int m = 16; m >= 1; m >>= 1) l += __shfl_xor_sync(kAll, l, m);
-          eloss += l;
-        }
+        if (want && trank == 0 && warp == 0) eloss += minibatch_loss(item_loss, n_items, lane);
         if (s1 > s0) team_sync();  // combined split rows are staged before the update reads them
         update_rows<kBF16>(a.xm, a.xb, stage, (G.voff + base) * D, rows * D, trank * blockDim.x + threadIdx.x,
                            nct * blockDim.x);  // algo.hpp:651-666

@@ -154,8 +154,8 @@ int de_minibatch_noalloc(int64_t n, const int32_t *rowptr, const int32_t *col, i
  * (cpp/dist_embed.cpp:334-344 builds one EmbeddingAlgo and calls
  * algo_force2_vec_ns once); each graph here follows that same one-rank step
  * (cpp/algo/algo.hpp:164-192) with its own sampler seeds (epoch + batch), as if
- * it ran alone.  One CTA ("team") owns a graph for all its epochs; teams take
- * graphs largest first.  dim is 32, 64 or 128; opts->precision picks FP32
+ * it ran alone.  A team (one CTA, or the CTAs of a cluster) owns a graph for all its
+ * epochs; teams take graphs largest first.  dim is 32, 64 or 128; opts->precision picks FP32
  * storage or BF16 storage with an FP32 master copy; opts->edge_cap (0: 32) is the
  * CSR entries of one work item, up to 4096. */
 typedef struct de_batch de_batch;
@@ -172,7 +172,8 @@ int de_batch_get_embeddings_f32(de_batch *b, int32_t graph, float *x);
 /* Team shape.  Two kernel families run the same step:
  *   DE_BATCH_REGISTER  work items read their rows into registers; a warp runs
  *                      vertices_per_warp (1, 2 or 4) items at once on 32, 16 or 8
- *                      lanes; team_warps 4, 8, 16 or 32; edge_cap 1..4096
+ *                      lanes; team_warps 4, 8, 16 or 32; edge_cap 1..4096; a team
+ *                      is 1, 2, 4 or 8 CTAs, whichever suits the graphs
  *   DE_BATCH_STAGED    every warp stages the rows of its next stages-1 chunks in
  *                      shared memory with 16-byte asynchronous copies; a pair is
  *                      computed by dim/8 lanes; team_warps 2..16; edge_cap 1..32
@@ -189,7 +190,7 @@ int de_batch_get_embeddings_f32(de_batch *b, int32_t graph, float *x);
 typedef struct de_batch_shape {
   int32_t kernel;            /* DE_BATCH_*                                   */
   int32_t vertices_per_warp; /* register kernel                              */
-  int32_t team_warps;        /* warps per team (one CTA per team)            */
+  int32_t team_warps;        /* warps of a CTA                               */
   int32_t edge_cap;          /* CSR entries per work item                    */
   int32_t pairs;             /* staged kernel: warp steps in flight          */
   int32_t stages;            /* staged kernel                                */
