@@ -104,7 +104,7 @@ KernelPick pick_kernel(int dim, bool bf16, const de_batch_shape &s, int ns = 0) 
     }
     return 0;
   };
-  k.fn = pick_staged(dim, bf16, s.pairs, s.stages, k.ctas);
+  k.fn = pick_staged(dim, bf16, s.pairs, s.stages, k.ctas > 1);
   // the column-id buffers where they fit; without them the kernel reads the ids
   // from global memory one chunk ahead
   k.stage_ids = smem_of(1) <= kStagedSmemMax ? 1 : 0;
@@ -315,13 +315,59 @@ int register_ctas(const de_batch *b, const de_batch_shape &s, int resident) {
   return best;
 }
 
-int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape) {
+// The graphs that clusters of `ctas` CTAs train together (the first n_big of b->order):
+// those above 0.6 of the balanced share of one of `teams` CTAs.
+int staged_big_graphs(const de_batch *b, const std::vector<double> &w, double total_w, int teams) {
+  int n = 0;
+  while (n < b->n_graphs && w[b->order[n]] > 0.6 * total_w / teams) ++n;
+  return n;
+}
+
+// CTAs to a cluster of the staged kernel, `from` (the shape's team_ctas) to 8,
+// whichever ends first: clusters take the big graphs, then their CTAs the others one
+// each.  STAGED_MODEL
+int staged_ctas(const de_batch *b, const std::vector<double> &w, double total_w, int from, int sms) {
+  constexpr double kFixedUs = 5.0, kShareUs = 5.7, kEntryUs = 0.0114;
+  auto cost = [&](int g, int ctas) {
+    return kFixedUs * b->ginfo[g].batches + (kShareUs * b->ginfo[g].batches + kEntryUs * double(b->nnz[g])) / ctas;
+  };
+  typedef std::priority_queue<double, std::vector<double>, std::greater<double>> Free;  // when each is free
+  int best = from;
+  double best_us = -1;
+  for (int ctas = from; ctas <= 8; ctas *= 2) {
+    const int clusters = sms / ctas;
+    if (clusters < 1) break;
+    const int big = staged_big_graphs(b, w, total_w, clusters * ctas);
+    Free cl, one;
+    for (int c = 0; c < clusters; ++c) cl.push(0.0);
+    double end = 0;
+    for (int i = 0; i < big; ++i) {
+      const double us = cl.top() + cost(b->order[i], ctas);
+      cl.pop();
+      cl.push(us);
+      end = std::max(end, us);
+    }
+    for (; !cl.empty(); cl.pop())
+      for (int c = 0; c < ctas; ++c) one.push(cl.top());
+    for (int i = big; i < b->n_graphs; ++i) {
+      const double us = one.top() + cost(b->order[i], 1);
+      one.pop();
+      one.push(us);
+      end = std::max(end, us);
+    }
+    if (best_us < 0 || end < best_us) best = ctas, best_us = end;
+  }
+  return best;
+}
+
+int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape, const std::vector<double> &w, double total_w) {
   int per_sm = 0, sms = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.block, k.smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || sms < 1) sms = 1;
   const bool reg = shape.kernel == DE_BATCH_REGISTER;
   if (reg) k.ctas = register_ctas(b, shape, per_sm * sms);
+  else if (k.ctas > 1) k.ctas = staged_ctas(b, w, total_w, k.ctas, per_sm * sms);
   if (k.ctas == 1) return std::min(per_sm * sms, b->n_graphs);
   // clusters of k.ctas CTAs: as many as can be resident at once (a cluster sits in one GPC)
   cudaLaunchConfig_t cfg{};
@@ -340,9 +386,7 @@ int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape) {
     cudaGetLastError();
     clusters = std::max(1, per_sm * sms / k.ctas);
   }
-  // a register team of several CTAs takes one graph; the CTAs of a staged one take
-  // the smaller graphs alone
-  return k.ctas * std::min(clusters, reg ? b->n_graphs : (b->n_graphs + k.ctas - 1) / k.ctas);
+  return k.ctas * std::min(clusters, b->n_graphs);
 }
 
 // Everything of a run except the launch: schedule, negatives, rates, team staging
@@ -400,12 +444,8 @@ int prepare_batched(de_batch *b, int epochs, int B, int ns, const double *lr, co
     total_w += w[g];
   }
   std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) { return w[x] > w[y]; });
-  const int teams = teams_for(b, k, shape);
-  // with staged teams of several CTAs the graphs above 0.6 of the balanced share of
-  // one CTA are trained by a whole cluster
-  b->n_big = 0;
-  if (k.ctas > 1 && shape.kernel != DE_BATCH_REGISTER)
-    while (b->n_big < b->n_graphs && w[b->order[b->n_big]] > 0.6 * total_w / teams) ++b->n_big;
+  const int teams = teams_for(b, k, shape, w, total_w);
+  b->n_big = k.ctas > 1 && shape.kernel != DE_BATCH_REGISTER ? staged_big_graphs(b, w, total_w, teams) : 0;
   BCUDA(b, cudaMemcpyAsync(b->d_order, b->order.data(), b->order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                            b->stream));
   BCUDA(b, cudaStreamSynchronize(b->stream));  // the host vectors go away on return

@@ -196,8 +196,9 @@ typedef struct de_batch_shape {
   int32_t stages;            /* staged kernel                                */
   int32_t team_ctas;         /* staged kernel: 2 or 4 = the largest graphs    */
                              /* are trained by the CTAs of a cluster of that  */
-                             /* size together (the rest one per CTA); 0 or 1  */
-                             /* = one CTA each                                */
+                             /* size together, or of up to 8 CTAs where few   */
+                             /* graphs leave SMs idle (the rest one per CTA); */
+                             /* 0 or 1 = one CTA each                         */
 } de_batch_shape;
 int de_batch_set_shape(de_batch *b, const de_batch_shape *shape);
 int de_batch_get_shape(const de_batch *b, de_batch_shape *shape);

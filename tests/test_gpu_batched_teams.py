@@ -30,11 +30,13 @@ def train(graphs, x0s, dim, precision, shape, batch, ns):
 
 
 REGISTER = dict(kernel="register", vertices_per_warp=2, team_warps=16, edge_cap=16)
+STAGED = dict(kernel="staged", team_warps=8, edge_cap=8, pairs=2, stages=3, team_ctas=2)
 
 
 @pytest.mark.parametrize("dim,precision,shape,batch,ns", [
     (32, "fp32", None, 100, 5), (32, "fp32", REGISTER, 37, 0), (64, "fp32", None, 256, 9), (64, "bf16", None, 100, 5),
-    (128, "fp32", None, 64, 33), (128, "bf16", REGISTER, 300, 3)])
+    (128, "fp32", None, 64, 33), (128, "bf16", REGISTER, 300, 3), (32, "fp32", STAGED, 100, 5),
+    (64, "bf16", STAGED, 256, 9), (128, "fp32", STAGED, 37, 0)])
 def test_alone_and_among_many(dim, precision, shape, batch, ns):
     big = gg.rmat_csr_n(700, 6, seed=dim)[1:]
     assert (np.diff(big[0]) == 0).any() and np.diff(big[0]).max() > 33
