@@ -237,20 +237,18 @@ cudaError_t launch_sparse_finalize(double *x64, int64_t count, cudaStream_t s);
 cudaError_t launch_f64_to_f32(const double *src, float *dst, int64_t count, cudaStream_t s);
 cudaError_t launch_f32_to_f64(const float *src, double *dst, int64_t count, cudaStream_t s);
 constexpr int kPlainWarps = 4;      // warps per CTA of the plain batch kernel
-constexpr int kPlainMinBlocks = 8;  // resident CTAs per SM the register budget targets (one wave of
-                                    // work items at minibatch 4096: 152 x 8 x 4 warps)
 // Warps to a work item of the FP32 plain form.  Several shorten the chain of a row
-// as long as the minibatch's warps then still run at once (152 SMs x 32 resident
-// warps, 16 at dim 256).  Measured crossings, in items of a minibatch: four against
-// two warps at 800 to 1,000 for every dim (kNN-20k, dim 128: 540 items 4.5 against
-// 5.2 us, 1,080 items 6.2 against 6.5, at dim 64 5.8 against 5.6); two against one
-// at about 2,500 (2,150 items 7.9 against 9.1 us, 3,200 items 11.1 against 10.5) and
-// at dim 256 at 1,600 to 2,000 (1,600 items 10.1 against 10.4 us, 2,150 items 13.9
-// against 12.1).
-constexpr int kTeam4MaxItems = 152 * 6;
-constexpr int team2_max_items(int dim) { return 152 * (dim >= 256 ? 12 : 16); }
+// as long as the minibatch's warps then still run at once (152 SMs x 24 resident
+// warps, 16 at dim 256).  Measured crossings, in items of a minibatch (microseconds a
+// minibatch): four against two warps at 600 to 850 (kNN-20k, dim 128: 609 items 4.4
+// against 4.5, 1,060 items 6.1 against 5.1) and not at all at dim 32, where a group of
+// eight pairs is one step; two against one at 1,750 to 2,200 for dim 64 and 128 (dim
+// 128: 1,625 items 5.9 against 7.0, 2,438 items 9.8 against 8.6) and at 1,300 to 1,900
+// for dim 32 and 256 (dim 256: 1,283 items 7.3 against 8.4, 2,031 items 10.7 against 9.3).
 constexpr int plain_team_warps(int dim, int n_items) {
-  return n_items <= kTeam4MaxItems ? 4 : n_items <= team2_max_items(dim) ? 2 : 1;
+  const int four = dim == 32 ? 0 : 152 * 4;
+  const int two = dim == 64 || dim == 128 ? 152 * 12 : 152 * 10;
+  return n_items <= four ? 4 : n_items <= two ? 2 : 1;
 }
 constexpr int kMaxEdgeCap = 32;     // CSR entries per work item: one per lane
 

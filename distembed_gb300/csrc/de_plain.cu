@@ -2,15 +2,14 @@
 //
 // One launch per minibatch.  A warp owns one work item (a row, or an edge-capped
 // piece of a high-degree row); items are sorted by decreasing cost so the block
-// scheduler hands out the long ones first.  Each lane holds dim/32 components of
-// a row, so a neighbour row is one coalesced 128-bit load per lane at dim 128.
-// Eight neighbour rows are in flight per warp; their eight squared distances are
-// reduced together (9 shuffles), each lane turns one of them into the
-// t-distribution coefficient and the coefficients are broadcast back (8
-// shuffles), then every lane clips and accumulates its components
-// (cpp/algo/algo.hpp:531-582).  The repulsive pass over the minibatch's shared
-// negatives (algo.hpp:594-647) and the update (algo.hpp:651-666) are fused into
-// the same pass.
+// scheduler hands out the long ones first.  The pairs of an item are its CSR entries
+// (cpp/algo/algo.hpp:531-582) and then, on a row's first piece, the minibatch's shared
+// negatives (algo.hpp:594-647): one sequence, each lane holding one pair's other row.
+// At dim 128 and 256 a warp holds a row, eight or four rows are in flight, their
+// squared distances are reduced together, each lane turns one of them into the
+// t-distribution coefficient and the coefficients are broadcast back; below, a pair is
+// computed by dim/8 lanes and a warp takes four or eight pairs a step.  The update
+// (algo.hpp:651-666) is fused into the same pass.
 //
 // Within a minibatch the reference reads only pre-minibatch values (the update
 // is applied after both passes), and minibatch j+1 must see minibatch j's update
@@ -49,51 +48,182 @@ __device__ __forceinline__ const float *row_ptr(const PlainBatchArgs &a, int n, 
   return off < unsigned(a.prev2_rows) ? a.S_prev2 + size_t(off) * D : a.X + size_t(n) * D;
 }
 
-// Gathers up to U rows named by lanes [k, k+U) of `ids` (one id per lane, -1 =
-// none) and applies their forces.  Missing rows get xi (zero force).
-template <int D, int U, bool kAttract, bool kAfterWait>
-__device__ __forceinline__ void force_group(const PlainBatchArgs &a, Frag<D> &acc, const Frag<D> &xi, int ids,
-                                            int k, float lr, float bound, bool want_loss, float &loss,
-                                            int lane) {
-  Frag<D> xn[U];
-  unsigned mask = 0;
+// Layout of a pair: LP lanes hold a row, C components each, G pairs a warp step and S
+// steps' rows in flight.  Lane gl of a pair holds components [4 gl, 4 gl + 4) and, with
+// C = 8, [D/2 + 4 gl, D/2 + 4 gl + 4): 128-bit loads, each contiguous over the lanes.
+// Below dim 128 a row is too short for a warp; at dim 128 two pairs a step measured
+// slower than one (R-MAT of 2^20 vertices, B = 4096: 18.3 against 15.0 us a
+// minibatch, at dim 64 11.9 against 12.6, dim 32 9.2 against 11.7).
+template <int D>
+struct Lay {
+  static constexpr int LP = D >= 128 ? 32 : D / 8, G = 32 / LP, C = D / LP;
+  static constexpr int S = D == 128 ? 8 : D == 256 ? 4 : 2;
+};
+template <int D>
+struct LaneRow {
+  float v[Lay<D>::C];
+  __device__ __forceinline__ void zero() {
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int n = __shfl_sync(kFull, ids, k + u);
-    if (n >= 0) {
-      if (kAfterWait) load_cg(xn[u], row_ptr<true>(a, n, D), lane);
-      else load_nc(xn[u], row_ptr<false>(a, n, D), lane);
-      mask |= 1u << u;
-    } else {
-      xn[u] = xi;
-    }
+    for (int t = 0; t < Lay<D>::C; ++t) v[t] = 0.f;
   }
-  if (mask) pair_forces<D, U, kAttract>(acc, xi, xn, mask, lr, bound, want_loss, loss, lane);
+};
+
+// Resident CTAs per SM the registers are held to.  One warp an item: 64 registers
+// spill at dim 128 (measured against 72, R-MAT of 2^20 vertices, B = 4096: 14.5 against
+// 13.6 us a minibatch) and pay below (dim 64: 10.5 against 11.0).  Several warps an
+// item do not fill the GPU, so they take 80.
+template <int D>
+constexpr int kMinBlocks = D >= 256 ? 4 : D == 128 ? 7 : 8;
+template <int D>
+constexpr int kTeamMinBlocks = D >= 256 ? 4 : 6;
+
+// How a row is read: kFinal, rows that no launch in flight writes (read-only path);
+// kStaged, rows of minibatch j-1 written by the launch before (L2); kShared, shared
+// memory or kFinal rows through generic addresses.
+enum RowRead { kFinal, kStaged, kShared };
+template <int D, RowRead kRead>
+__device__ __forceinline__ void load_lanes(LaneRow<D> &f, const float *row, int gl) {
+  const float4 *p = reinterpret_cast<const float4 *>(row) + gl;
+#pragma unroll
+  for (int h = 0; h < Lay<D>::C / 4; ++h, p += D / 8) {
+    const float4 t = kRead == kFinal ? __ldg(p) : kRead == kStaged ? __ldcg(p) : *p;
+    f.v[4 * h] = t.x; f.v[4 * h + 1] = t.y; f.v[4 * h + 2] = t.z; f.v[4 * h + 3] = t.w;
+  }
 }
 
-// Forces of the ids held by the warp's lanes (-1 = none), U at a time; a last
-// group of at most U/2 entries runs as a group of U/2.
-template <int D, int U, bool kAttract, bool kAfterWait>
-__device__ __forceinline__ void force_lanes(const PlainBatchArgs &a, Frag<D> &acc, const Frag<D> &xi, int ids,
-                                            int cnt, float lr, float bound, bool want_loss, float &loss,
-                                            int lane) {
-  int k = 0;
-  for (; k + U / 2 < cnt; k += U)
-    force_group<D, U, kAttract, kAfterWait>(a, acc, xi, ids, k, lr, bound, want_loss, loss, lane);
-  if (k < cnt) force_group<D, U / 2, kAttract, kAfterWait>(a, acc, xi, ids, k, lr, bound, want_loss, loss, lane);
+// Stores of lanes [0, LP), which hold a whole row.
+template <int D, bool kCg>
+__device__ __forceinline__ void store_lanes(const LaneRow<D> &f, float *row, int lane) {
+  if (lane >= Lay<D>::LP) return;
+  float4 *p = reinterpret_cast<float4 *>(row) + lane;
+#pragma unroll
+  for (int h = 0; h < Lay<D>::C / 4; ++h, p += D / 8) {
+    const float4 t = make_float4(f.v[4 * h], f.v[4 * h + 1], f.v[4 * h + 2], f.v[4 * h + 3]);
+    if constexpr (kCg) __stcg(p, t);
+    else *p = t;
+  }
 }
 
-// Split rows: two-level, fixed-order combine of the parts; true on the warp that
-// ends up with the row's sum (every warp of an unsplit row).
+// The lane groups' sums of a row added up (fixed order), on every lane.
+template <int D>
+__device__ __forceinline__ void sum_groups(LaneRow<D> &acc) {
+#pragma unroll
+  for (int m = Lay<D>::LP; m < 32; m <<= 1)
+#pragma unroll
+    for (int t = 0; t < Lay<D>::C; ++t) acc.v[t] += __shfl_xor_sync(kFull, acc.v[t], m);
+}
+
+// What an item's pairs share.
+struct PairCtx {
+  float lr, bound, clip_r;
+  bool want_loss;
+  __device__ __forceinline__ PairCtx(const PlainBatchArgs &a, int epoch)
+      : lr(a.lr[epoch]), bound(a.bound), want_loss(a.compute_loss != 0) {
+    // |c (x_d - n_d)| <= |c| sqrt(r): 2 sqrt(r) / (1 + r) <= 1 for attraction, less
+    // than 2 / sqrt(r) for repulsion.  So the clip (algo.hpp:65-72) is the identity at
+    // bound >= 1 and r >= clip_r = 4 / bound^2 (and 3 % more for rounding).
+    clip_r = bound >= 1.0f ? 4.12f / (bound * bound) : __int_as_float(0x7f800000);
+  }
+};
+
+// S steps of pairs [k0, k0 + S G) of a window of 32: lane k of `rows` holds pair k's
+// other row.  Bit k of vm: pair k counts, of rm: it counts and repels.  The row of a
+// pair that does not count is x_i's own, whose (attractive) force is exactly 0.
+// Attractive: c = -2/(1+r); repulsive: c = 2/((r+1e-6)(1+r)) (algo.hpp:573, 626/641).
+template <int D, int S, RowRead kRead>
+__device__ __forceinline__ void pair_steps(LaneRow<D> &acc, const LaneRow<D> &xi, const float *rows, unsigned vm,
+                                           unsigned rm, int k0, const PairCtx &c, float &loss, int lane) {
+  constexpr int LP = Lay<D>::LP, G = Lay<D>::G, C = Lay<D>::C;
+  const int q = G > 1 ? lane / LP : 0, gl = G > 1 ? lane % LP : lane;
+  LaneRow<D> x[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const float *row = reinterpret_cast<const float *>(
+        __shfl_sync(kFull, reinterpret_cast<unsigned long long>(rows), k0 + s * G + q));
+    load_lanes<D, kRead>(x[s], row, gl);
+  }
+  float r[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    float2 p = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < C; t += 2) {
+      const float2 d = sub2(make_float2(xi.v[t], xi.v[t + 1]), make_float2(x[s].v[t], x[s].v[t + 1]));
+      x[s].v[t] = d.x;
+      x[s].v[t + 1] = d.y;
+      p = __ffma2_rn(d, d, p);
+    }
+    r[s] = p.x + p.y;
+  }
+  bool may_clip = false;
+  // coefficient and loss term of pair k at squared distance rr; the term is added on
+  // one lane of the pair
+  auto coefficient = [&](float rr, int k, bool adds) -> float {
+    const bool at = !((rm >> k) & 1u);
+    const float one = 1.0f + rr, eps = rr + 1e-6f;
+    may_clip |= rr < c.clip_r && (!at || c.bound < 1.0f);
+    if (c.want_loss && adds && ((vm >> k) & 1u)) loss += at ? log1pf(rr) : logf(one / eps);
+    return __fdividef(at ? -2.0f : 2.0f, at ? one : eps * one);
+  };
+  float cf[S];
+  if constexpr (G == 1) {
+    // S sums over the whole warp at once; lane group v holds pair v's
+    constexpr int L = Log2<S>::value;
+    const float rr = multi_warp_sum<S>(r, lane);
+    const int v = (lane >> (5 - L)) & (S - 1);
+    const float cv = coefficient(rr, k0 + v, (lane & ((32 >> L) - 1)) == 0);
+#pragma unroll
+    for (int s = 0; s < S; ++s) cf[s] = __shfl_sync(kFull, cv, s << (5 - L));
+  } else {
+#pragma unroll
+    for (int m = LP / 2; m >= 1; m >>= 1)
+#pragma unroll
+      for (int s = 0; s < S; ++s) r[s] += __shfl_xor_sync(kFull, r[s], m);
+#pragma unroll
+    for (int s = 0; s < S; ++s) cf[s] = coefficient(r[s], k0 + s * G + q, gl == 0);
+  }
+  if (!__any_sync(kFull, may_clip)) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const float lc = c.lr * cf[s];
+#pragma unroll
+      for (int t = 0; t < C; t += 2) {
+        const float2 o = __ffma2_rn(make_float2(lc, lc), make_float2(x[s].v[t], x[s].v[t + 1]),
+                                    make_float2(acc.v[t], acc.v[t + 1]));
+        acc.v[t] = o.x;
+        acc.v[t + 1] = o.y;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+#pragma unroll
+      for (int t = 0; t < C; ++t) acc.v[t] = fmaf(c.lr, clip(x[s].v[t] * cf[s], c.bound), acc.v[t]);
+  }
+}
+
+// Every pair of a window of 32, S steps at a time and half as many at its end.
+template <int D, RowRead kRead>
+__device__ __forceinline__ void pair_window(LaneRow<D> &acc, const LaneRow<D> &xi, const float *rows, unsigned vm,
+                                            unsigned rm, const PairCtx &c, float &loss, int lane) {
+  constexpr int S = Lay<D>::S, kChunk = S * Lay<D>::G;
+  const int end = 32 - __clz(vm);
+  for (int k = 0; k < end; k += kChunk) {
+    if (((vm >> k) & (kFull >> (32 - kChunk))) == 0) continue;
+    if (end - k > kChunk / 2) pair_steps<D, S, kRead>(acc, xi, rows, vm, rm, k, c, loss, lane);
+    else pair_steps<D, S / 2, kRead>(acc, xi, rows, vm, rm, k, c, loss, lane);
+  }
+}
+
+// Split rows: two-level, fixed-order combine of the parts; the partial is in slot
+// it.first_slot + it.part.  True on the warp that ends up with the row's sum, in acc.
 template <int D>
 __device__ __forceinline__ bool combine_parts(Frag<D> &acc, const WorkItem &it, float *slots, int32_t *counters,
                                               int lane) {
-  if (it.nparts <= 1) return true;
   const int P = it.nparts;
   const int g = it.part / kCombineGroup;
   const int ng = (P + kCombineGroup - 1) / kCombineGroup;
   const int gsize = min(kCombineGroup, P - g * kCombineGroup);
-  store<D, true>(acc, slots + size_t(it.first_slot + it.part) * D, lane);
   bool owner = arrive_last(counters + it.counter + g, gsize, lane);
   if (owner) {
     sum_slots(acc, slots + size_t(it.first_slot + g * kCombineGroup) * D, gsize, lane);
@@ -106,47 +236,40 @@ __device__ __forceinline__ bool combine_parts(Frag<D> &acc, const WorkItem &it, 
   return owner;
 }
 
-// A row held in shared memory, in the Frag layout.
+// The item's update: a whole row's new value staged (algo.hpp:651-666), or the part
+// combined with the row's others and the row staged by the last of them.
 template <int D>
-__device__ __forceinline__ void load_smem(Frag<D> &f, const float *row, int lane) {
-  if constexpr (D == 32) {
-    f.v[0] = row[lane];
-  } else if constexpr (D == 64) {
-    const float2 t = reinterpret_cast<const float2 *>(row)[lane];
-    f.v[0] = t.x; f.v[1] = t.y;
-  } else {
-    const float4 t = reinterpret_cast<const float4 *>(row)[lane];
-    f.v[0] = t.x; f.v[1] = t.y; f.v[2] = t.z; f.v[3] = t.w;
-    if constexpr (D == 256) {
-      const float4 u = reinterpret_cast<const float4 *>(row)[32 + lane];
-      f.v[4] = u.x; f.v[5] = u.y; f.v[6] = u.z; f.v[7] = u.w;
-    }
-  }
-}
-
-// Repulsive forces of staged negatives k0 .. k0+V-1 (rows in shared memory;
-// draws whose bit in `staged` is clear are left out).
-template <int D, int V>
-__device__ __forceinline__ void staged_group(Frag<D> &acc, const Frag<D> &xi, const float *negsm, unsigned staged,
-                                             int k0, int ns, float lr, float bound, bool want_loss, float &loss,
-                                             int lane) {
-  Frag<D> xn[V];
-  unsigned mask = 0;
+__device__ __forceinline__ void finish_item(const PlainBatchArgs &a, const WorkItem &it, const LaneRow<D> &xi,
+                                            LaneRow<D> &acc, int lane) {
+  float *out = a.S_cur + size_t(it.row) * D;
+  if (it.nparts <= 1) {
 #pragma unroll
-  for (int u = 0; u < V; ++u) {
-    const int k = k0 + u;
-    if (k < ns && ((staged >> k) & 1u)) {
-      load_smem(xn[u], negsm + k * D, lane);
-      mask |= 1u << u;
-    } else {
-      xn[u] = xi;
-    }
+    for (int t = 0; t < Lay<D>::C; ++t) acc.v[t] = xi.v[t] + acc.v[t];
+    store_lanes<D, false>(acc, out, lane);
+    return;
   }
-  if (mask) pair_forces<D, V, false>(acc, xi, xn, mask, lr, bound, want_loss, loss, lane);
+  store_lanes<D, true>(acc, a.P + size_t(it.first_slot + it.part) * D, lane);
+  Frag<D> sum, x;
+  if (!combine_parts<D>(sum, it, a.P, a.counters, lane)) return;
+  load_nc(x, a.X + size_t(a.base + it.row) * D, lane);
+#pragma unroll
+  for (int t = 0; t < Frag<D>::N; ++t) sum.v[t] = x.v[t] + sum.v[t];
+  store<D, false>(sum, out, lane);
 }
 
-template <int D, int U>
-__global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBlocks)
+// Rows of minibatch j-1: staging buffer -> X.  Until the next launch passes
+// its wait, every reader takes these rows from the staging buffer.
+template <int D>
+__device__ __forceinline__ void copy_back(const PlainBatchArgs &a, int lane, int gw, int total_w) {
+  for (int r = gw; r < a.prev_rows; r += total_w) {
+    Frag<D> t;
+    load_cg(t, a.S_prev + size_t(r) * D, lane);
+    store<D, false>(t, a.X + size_t(a.prev_base + r) * D, lane);
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kPlainWarps * 32, kMinBlocks<D>)
     plain_batch_kernel(const PlainBatchArgs a) {
   extern __shared__ __align__(16) float negsm[];  // stage_negs: [ns, D] rows of the minibatch's draws
   __shared__ __align__(8) uint64_t negbar;
@@ -154,7 +277,6 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
   const int lane = threadIdx.x & 31;
   const int gw = blockIdx.x * kPlainWarps + (threadIdx.x >> 5);
   const int total_w = gridDim.x * kPlainWarps;
-  const bool want_loss = a.compute_loss != 0;
 
   // an epoch's first minibatch reads what the launch before it writes
   if (a.first) pdl_wait();
@@ -162,27 +284,32 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
   WorkItem it{};
   if (has_item) it = a.items[gw];
   const int epoch = a.epoch[0];
-  const float lr = a.lr[epoch];
-  const float bound = a.bound;
+  const PairCtx c(a, epoch);
   const int skip = a.skip_last ? a.n - 1 : -1;  // edges into n-1 are dropped (algo.hpp:399-405, 538)
-  // this item's CSR entries, one per lane (at most 32)
-  const int cnt = has_item ? it.e_end - it.e_begin : 0;
-  int ids = -1;
-  if (lane < cnt) {
-    ids = __ldg(a.col + it.e_begin + lane);
-    if (ids == skip) ids = -1;
-  }
-  const bool defer = ids >= 0 && in_prev(a, ids);
+  const int cnt = it.e_end - it.e_begin;
   // the repulsive pass of a row is done by its part 0
   const int rep_rows = (a.quirks && epoch + a.epoch[1] > 0) ? a.last_batch_size : a.rows;
-  const bool repulse = has_item && it.part == 0 && it.row < rep_rows;
+  const int total = cnt + (has_item && it.part == 0 && it.row < rep_rows ? a.ns : 0);
   const int32_t *negs = a.negs + (size_t(epoch) * a.batches + a.batch_id) * a.ns;
+  // the other row of the item's pair k0 + lane: its CSR entries, then the draws; -1 = none
+  auto fetch = [&](int k0) -> int {
+    const int k = k0 + lane;
+    int id = -1;
+    if (k < cnt) {
+      id = __ldg(a.col + it.e_begin + k);
+      if (id == skip) id = -1;
+    } else if (k < total) {
+      id = __ldg(negs + k - cnt);
+      if (id >= a.n) id = -1;  // a draw equal to n contributes nothing
+    }
+    return id;
+  };
 
   // Staged negatives: bit k of `staged`: draw k is a vertex outside minibatch j-1
   // (final before the wait), copied by one thread of the CTA into row k of negsm
   // with bulk asynchronous copies; the CTA waits (bounded) on one barrier.
-  unsigned staged = 0;
   if (a.stage_negs) {
+    unsigned staged = 0;
     for (int k = 0; k < a.ns; ++k) {
       const int nid = __ldg(negs + k);
       if (nid >= 0 && nid < a.n && !in_prev(a, nid)) staged |= 1u << k;
@@ -198,70 +325,45 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
           bulk_g2s(smem_u32(negsm + k * D), row_ptr<false>(a, __ldg(negs + k), D), D * 4u, bar);
     }
     __syncthreads();
-    if (!mbar_wait(bar, 0, &negerr)) {
-      if (lane == 0) atomicExch(a.err, 1);
-      staged = 0;  // results of this launch are invalid; the host reports the error
-    }
+    // after a timeout the results of this launch are invalid; the host reports the error
+    if (!mbar_wait(bar, 0, &negerr) && lane == 0) atomicExch(a.err, 1);
   }
 
   float loss = 0.f;  // this item's loss terms (FP32); the epoch sum is FP64
-  Frag<D> xi, acc;
+  const float *const own = a.X + size_t(a.base + it.row) * D;
+  LaneRow<D> xi, acc;
   acc.zero();
-  if (has_item) {
-    load_nc(xi, a.X + size_t(a.base + it.row) * D, lane);
-    // ---- before the wait: forces whose other row is final (CSR order, then draw order)
-    force_lanes<D, U, true, false>(a, acc, xi, defer ? -1 : ids, cnt, lr, bound, want_loss, loss, lane);
-    if (repulse && a.stage_negs) {
-      // the staged rows in draw order, grouped as force_lanes groups them (so the
-      // arithmetic, and the result, equal the unstaged path's)
-      int k0 = 0;
-      for (; k0 + U / 2 < a.ns; k0 += U)
-        staged_group<D, U>(acc, xi, negsm, staged, k0, a.ns, lr, bound, want_loss, loss, lane);
-      if (k0 < a.ns) staged_group<D, U / 2>(acc, xi, negsm, staged, k0, a.ns, lr, bound, want_loss, loss, lane);
-    } else if (repulse)
-      for (int k0 = 0; k0 < a.ns; k0 += 32) {
-        const int kc = min(32, a.ns - k0);
-        int nid = lane < kc ? __ldg(negs + k0 + lane) : -1;
-        if (nid >= a.n || (nid >= 0 && in_prev(a, nid))) nid = -1;  // a draw equal to n contributes nothing
-        force_lanes<D, U, false, false>(a, acc, xi, nid, kc, lr, bound, want_loss, loss, lane);
-      }
-  }
-
-  pdl_wait();
-  pdl_trigger();
-
-  if (has_item) {
-    // ---- after the wait: forces into minibatch j-1
-    if (__any_sync(kFull, defer))
-      force_lanes<D, U, true, true>(a, acc, xi, defer ? ids : -1, cnt, lr, bound, want_loss, loss, lane);
-    if (repulse && a.prev_rows > 0)
-      for (int k0 = 0; k0 < a.ns; k0 += 32) {
-        const int kc = min(32, a.ns - k0);
-        int nid = lane < kc ? __ldg(negs + k0 + lane) : -1;
-        if (!(nid >= 0 && nid < a.n && in_prev(a, nid))) nid = -1;
-        if (__any_sync(kFull, nid >= 0))
-          force_lanes<D, U, false, true>(a, acc, xi, nid, kc, lr, bound, want_loss, loss, lane);
-      }
-
-    const bool owner = combine_parts<D>(acc, it, a.P, a.counters, lane);
-    // ---- update, staged (algo.hpp:651-666)
-    if (owner) {
-      Frag<D> out;
-#pragma unroll
-      for (int t = 0; t < Frag<D>::N; ++t) out.v[t] = xi.v[t] + acc.v[t];
-      store<D, false>(out, a.S_cur + size_t(it.row) * D, lane);
+  int ids = fetch(0);
+  if (has_item) load_lanes<D, kFinal>(xi, own, lane % Lay<D>::LP);
+  // ---- before the wait: forces whose other row is final
+  for (int k0 = 0; k0 < total; k0 += 32) {
+    if (k0 > 0) ids = fetch(k0);
+    const bool now = ids >= 0 && !in_prev(a, ids);
+    const bool repels = now && k0 + lane >= cnt;
+    const unsigned vm = __ballot_sync(kFull, now), rm = __ballot_sync(kFull, repels);
+    const float *row = now ? row_ptr<false>(a, ids, D) : own;
+    if (a.stage_negs) {
+      if (repels) row = negsm + (k0 + lane - cnt) * D;
+      pair_window<D, kShared>(acc, xi, row, vm, rm, c, loss, lane);
+    } else {
+      pair_window<D, kFinal>(acc, xi, row, vm, rm, c, loss, lane);
     }
   }
-
-  // Rows of minibatch j-1: staging buffer -> X.  Until the next launch passes
-  // its wait, every reader takes these rows from the staging buffer.
-  for (int r = gw; r < a.prev_rows; r += total_w) {
-    Frag<D> t;
-    load_cg(t, a.S_prev + size_t(r) * D, lane);
-    store<D, false>(t, a.X + size_t(a.prev_base + r) * D, lane);
+  pdl_wait();
+  pdl_trigger();
+  // ---- after the wait: forces into minibatch j-1
+  for (int k0 = 0; a.prev_rows > 0 && k0 < total; k0 += 32) {
+    if (total > 32) ids = fetch(k0);
+    const bool late = ids >= 0 && in_prev(a, ids);
+    const unsigned vm = __ballot_sync(kFull, late), rm = __ballot_sync(kFull, late && k0 + lane >= cnt);
+    if (vm) pair_window<D, kStaged>(acc, xi, late ? row_ptr<true>(a, ids, D) : own, vm, rm, c, loss, lane);
   }
-
-  if (want_loss && has_item) {
+  if (has_item) {
+    sum_groups<D>(acc);
+    finish_item<D>(a, it, xi, acc, lane);
+  }
+  copy_back<D>(a, lane, gw, total_w);
+  if (c.want_loss && has_item) {
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) loss += __shfl_xor_sync(kFull, loss, m);
     if (lane == 0) a.loss_partial[a.loss_off + gw] = double(loss);
@@ -272,113 +374,105 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
 //
 // The same step with W warps to a work item.  A minibatch that does not fill the
 // GPU takes as long as the longest chain in it, and a warp alone goes through a
-// row's groups of U pairs one after another (each a load, 17 shuffles and a divide:
-// about 0.6 us).  Here an item's CSR entries and then its draws are cut into groups
-// of U, group q on warp q % W, so a row of 32 entries and its draws is two rounds at
-// W = 4 instead of five; the warps' sums are added in warp order through shared
-// memory.  Phases, staging ring and split rows as in plain_batch_kernel.  Measured,
-// microseconds a minibatch, one warp an item -> this: 20,000-vertex kNN graph, dim
-// 128: B = 64 6.4 -> 3.4, 256 6.7 -> 4.0, 1024 8.3 -> 6.5; dim 256, B = 256 7.9 ->
-// 4.3; R-MAT of 100,003 vertices, dim 64, B = 512 6.3 -> 4.8.  Eight warps an item,
-// or groups of four pairs, gain at most 6 % below 100 items and lose above 300.
-template <int D, int U, int W>
-__global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBlocks)
+// row's pairs chunk after chunk (a load, a reduction, a divide: about 0.6 us).  Here
+// an item's pairs are cut into groups of 8 (4 at dim 256), group q on warp q % W, so a
+// row of 32 entries and its draws is two rounds at W = 4 instead of five; the warps'
+// sums are added in warp order through shared memory.  Phases, staging ring and split
+// rows as in plain_batch_kernel.  Measured, microseconds a minibatch at one / two / four
+// warps an item: 20,000-vertex kNN graph, dim 128: B = 256 5.0 / 4.0 / 3.9, 1100 6.5 /
+// 5.5 / 6.8; dim 256, B = 256 6.7 / 5.1 / 4.1; R-MAT of 100,003 vertices, dim 64, B = 512
+// 5.1 / 4.5 / 5.0.  Eight warps an item, or groups of half the size, gained at most 6 %
+// below 100 items and lost above 300.
+template <int D, int W>
+__global__ void __launch_bounds__(kPlainWarps * 32, kTeamMinBlocks<D>)
     plain_team_kernel(const PlainBatchArgs a) {
-  constexpr int kTeams = kPlainWarps / W;  // items of a CTA
-  constexpr int kRounds = 32 / U;          // groups of a warp whose ids its lanes hold at once
+  constexpr int kTeams = kPlainWarps / W;      // items of a CTA
+  constexpr int kPairs = D >= 256 ? 4 : 8;     // pairs of a group
+  constexpr int kSteps = kPairs / Lay<D>::G;
+  constexpr int kGroups = 32 / kPairs;         // groups of a warp whose ids its lanes hold at once
   __shared__ float s_acc[kTeams][W - 1][D];
   __shared__ float s_loss[kTeams][W - 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int team = warp / W, tw = warp % W;
   const int item = blockIdx.x * kTeams + team;
-  const bool want_loss = a.compute_loss != 0;
   if (a.first) pdl_wait();  // as in plain_batch_kernel
   const bool has_item = item < a.n_items;
   WorkItem it{};
   if (has_item) it = a.items[item];
   const int epoch = a.epoch[0];
-  const float lr = a.lr[epoch], bound = a.bound;
+  const PairCtx c(a, epoch);
   const int skip = a.skip_last ? a.n - 1 : -1;  // edges into n-1 are dropped (algo.hpp:399-405, 538)
-  const int cnt = has_item ? it.e_end - it.e_begin : 0;
+  const int cnt = it.e_end - it.e_begin;
   // the repulsive pass of a row is done by its part 0
   const int rep_rows = (a.quirks && epoch + a.epoch[1] > 0) ? a.last_batch_size : a.rows;
+  const int total = cnt + (has_item && it.part == 0 && it.row < rep_rows ? a.ns : 0);
   const int32_t *negs = a.negs + (size_t(epoch) * a.batches + a.batch_id) * a.ns;
-  const int ge = (cnt + U - 1) / U;
-  const int groups = ge + (has_item && it.part == 0 && it.row < rep_rows ? (a.ns + U - 1) / U : 0);
-  // the other row of entry lane % U of this warp's group s + lane / U, -1 = none
-  auto fetch = [&](int s) -> int {
-    const int q = (s + lane / U) * W + tw, k = (q < ge ? q : q - ge) * U + lane % U;
+  const int groups = (total + kPairs - 1) / kPairs;
+  const int mine = groups > tw ? (groups - tw + W - 1) / W : 0;  // this warp's groups
+  // entry lane % kPairs of this warp's group s + lane / kPairs: its index among the
+  // item's pairs, and its other row (-1 = none)
+  auto entry = [&](int s) -> int { return ((s + lane / kPairs) * W + tw) * kPairs + lane % kPairs; };
+  auto fetch = [&](int k) -> int {
     int id = -1;
-    if (q < ge) {
-      if (k < cnt) id = __ldg(a.col + it.e_begin + k);
+    if (k < cnt) {
+      id = __ldg(a.col + it.e_begin + k);
       if (id == skip) id = -1;
-    } else if (q < groups) {
-      if (k < a.ns) id = __ldg(negs + k);
+    } else if (k < total) {
+      id = __ldg(negs + k - cnt);
       if (id >= a.n) id = -1;  // a draw equal to n contributes nothing
     }
     return id;
   };
-  const int mine = groups > tw ? (groups - tw + W - 1) / W : 0;  // this warp's groups
   float loss = 0.f;
-  Frag<D> xi, acc;
+  const float *const own = a.X + size_t(a.base + it.row) * D;
+  LaneRow<D> xi, acc;
   acc.zero();
-  int ids = mine > 0 ? fetch(0) : -1;
-  if (has_item) load_nc(xi, a.X + size_t(a.base + it.row) * D, lane);
+  int ids = mine > 0 ? fetch(entry(0)) : -1;
+  if (has_item) load_lanes<D, kFinal>(xi, own, lane % Lay<D>::LP);
   // ---- before the wait: forces whose other row is final
-  for (int s = 0; s < mine; s += kRounds) {
-    if (s > 0) ids = fetch(s);
-    const int now = ids >= 0 && in_prev(a, ids) ? -1 : ids;
-    for (int r = 0; r < kRounds && s + r < mine; ++r) {
-      if ((s + r) * W + tw < ge)
-        force_group<D, U, true, false>(a, acc, xi, now, r * U, lr, bound, want_loss, loss, lane);
-      else
-        force_group<D, U, false, false>(a, acc, xi, now, r * U, lr, bound, want_loss, loss, lane);
-    }
+  for (int s = 0; s < mine; s += kGroups) {
+    if (s > 0) ids = fetch(entry(s));
+    const bool now = ids >= 0 && !in_prev(a, ids);
+    const unsigned vm = __ballot_sync(kFull, now), rm = __ballot_sync(kFull, now && entry(s) >= cnt);
+    const float *row = now ? row_ptr<false>(a, ids, D) : own;
+    for (int r = 0; r < kGroups && s + r < mine; ++r)
+      if ((vm >> (r * kPairs)) & ((1u << kPairs) - 1))
+        pair_steps<D, kSteps, kFinal>(acc, xi, row, vm, rm, r * kPairs, c, loss, lane);
   }
   pdl_wait();
   pdl_trigger();
   // ---- after the wait: forces into minibatch j-1
-  for (int s = 0; a.prev_rows > 0 && s < mine; s += kRounds) {
-    if (mine > kRounds) ids = fetch(s);
-    const int late = ids >= 0 && in_prev(a, ids) ? ids : -1;
-    if (!__any_sync(kFull, late >= 0)) continue;
-    for (int r = 0; r < kRounds && s + r < mine; ++r) {
-      if ((s + r) * W + tw < ge)
-        force_group<D, U, true, true>(a, acc, xi, late, r * U, lr, bound, want_loss, loss, lane);
-      else
-        force_group<D, U, false, true>(a, acc, xi, late, r * U, lr, bound, want_loss, loss, lane);
-    }
+  for (int s = 0; a.prev_rows > 0 && s < mine; s += kGroups) {
+    if (mine > kGroups) ids = fetch(entry(s));
+    const bool late = ids >= 0 && in_prev(a, ids);
+    const unsigned vm = __ballot_sync(kFull, late), rm = __ballot_sync(kFull, late && entry(s) >= cnt);
+    const float *row = late ? row_ptr<true>(a, ids, D) : own;
+    for (int r = 0; vm != 0 && r < kGroups && s + r < mine; ++r)
+      if ((vm >> (r * kPairs)) & ((1u << kPairs) - 1))
+        pair_steps<D, kSteps, kStaged>(acc, xi, row, vm, rm, r * kPairs, c, loss, lane);
   }
-  if (want_loss) {
+  sum_groups<D>(acc);
+  if (c.want_loss) {
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) loss += __shfl_xor_sync(kFull, loss, m);
   }
-  // rows of minibatch j-1: staging buffer -> X, as in plain_batch_kernel
-  const int gw = blockIdx.x * kPlainWarps + warp, total_w = gridDim.x * kPlainWarps;
-  for (int r = gw; r < a.prev_rows; r += total_w) {
-    Frag<D> t;
-    load_cg(t, a.S_prev + size_t(r) * D, lane);
-    store<D, false>(t, a.X + size_t(a.prev_base + r) * D, lane);
-  }
+  copy_back<D>(a, lane, blockIdx.x * kPlainWarps + warp, gridDim.x * kPlainWarps);
   if (tw > 0) {
-#pragma unroll
-    for (int t = 0; t < Frag<D>::N; ++t) s_acc[team][tw - 1][t * 32 + lane] = acc.v[t];
+    store_lanes<D, false>(acc, s_acc[team][tw - 1], lane);
     if (lane == 0) s_loss[team][tw - 1] = loss;
   }
   __syncthreads();
   if (tw > 0 || !has_item) return;
 #pragma unroll
   for (int w = 0; w < W - 1; ++w) {
+    LaneRow<D> t;
+    load_lanes<D, kShared>(t, s_acc[team][w], lane % Lay<D>::LP);
 #pragma unroll
-    for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] += s_acc[team][w][t * 32 + lane];
+    for (int k = 0; k < Lay<D>::C; ++k) acc.v[k] += t.v[k];
     loss += s_loss[team][w];
   }
-  if (combine_parts<D>(acc, it, a.P, a.counters, lane)) {
-#pragma unroll
-    for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] = xi.v[t] + acc.v[t];
-    store<D, false>(acc, a.S_cur + size_t(it.row) * D, lane);
-  }
-  if (want_loss && lane == 0) a.loss_partial[a.loss_off + item] = double(loss);
+  finish_item<D>(a, it, xi, acc, lane);
+  if (c.want_loss && lane == 0) a.loss_partial[a.loss_off + item] = double(loss);
 }
 
 // SpMMAlgo::algo_spmm's step at one rank (cpp/algo/spmm.hpp:54-159):
@@ -389,7 +483,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : kPlainMinBloc
 // work item, U rows in flight; split rows are combined in piece order as in
 // plain_batch_kernel.
 template <int D, int U>
-__global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : (D == 128 ? 10 : kPlainMinBlocks))
+__global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : (D == 128 ? 10 : 8))
     spmm_kernel(const SpmmArgs a) {
   const int lane = threadIdx.x & 31;
   const int64_t gw = blockIdx.x * int64_t(kPlainWarps) + (threadIdx.x >> 5);
@@ -419,7 +513,11 @@ __global__ void __launch_bounds__(kPlainWarps * 32, D >= 256 ? 4 : (D == 128 ? 1
 #pragma unroll
       for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] = fmaf(a.lr, xn[u].v[t], acc.v[t]);
   }
-  const bool owner = combine_parts<D>(acc, it, P, counters, lane);
+  bool owner = true;
+  if (it.nparts > 1) {
+    store<D, true>(acc, P + size_t(it.first_slot + it.part) * D, lane);
+    owner = combine_parts<D>(acc, it, P, counters, lane);
+  }
   if (owner) store<D, false>(acc, a.Y + (size_t(j) * a.batch + it.row) * D, lane);
 }
 
@@ -530,27 +628,27 @@ cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, bool teams, boo
   const int grid = (a.n_items * w + kPlainWarps - 1) / kPlainWarps;
   if (w == 4) {
     switch (dim) {
-      case 32: return launch(plain_team_kernel<32, 8, 4>, grid, block, a, pdl, s);
-      case 64: return launch(plain_team_kernel<64, 8, 4>, grid, block, a, pdl, s);
-      case 128: return launch(plain_team_kernel<128, 8, 4>, grid, block, a, pdl, s);
-      case 256: return launch(plain_team_kernel<256, 4, 4>, grid, block, a, pdl, s);
+      case 32: return launch(plain_team_kernel<32, 4>, grid, block, a, pdl, s);
+      case 64: return launch(plain_team_kernel<64, 4>, grid, block, a, pdl, s);
+      case 128: return launch(plain_team_kernel<128, 4>, grid, block, a, pdl, s);
+      case 256: return launch(plain_team_kernel<256, 4>, grid, block, a, pdl, s);
       default: return cudaErrorInvalidValue;
     }
   }
   if (w == 2) {
     switch (dim) {
-      case 32: return launch(plain_team_kernel<32, 8, 2>, grid, block, a, pdl, s);
-      case 64: return launch(plain_team_kernel<64, 8, 2>, grid, block, a, pdl, s);
-      case 128: return launch(plain_team_kernel<128, 8, 2>, grid, block, a, pdl, s);
-      case 256: return launch(plain_team_kernel<256, 4, 2>, grid, block, a, pdl, s);
+      case 32: return launch(plain_team_kernel<32, 2>, grid, block, a, pdl, s);
+      case 64: return launch(plain_team_kernel<64, 2>, grid, block, a, pdl, s);
+      case 128: return launch(plain_team_kernel<128, 2>, grid, block, a, pdl, s);
+      case 256: return launch(plain_team_kernel<256, 2>, grid, block, a, pdl, s);
       default: return cudaErrorInvalidValue;
     }
   }
   switch (dim) {
-    case 32: return launch(plain_batch_kernel<32, 8>, grid, block, a, pdl, s, smem);
-    case 64: return launch(plain_batch_kernel<64, 8>, grid, block, a, pdl, s, smem);
-    case 128: return launch(plain_batch_kernel<128, 8>, grid, block, a, pdl, s, smem);
-    case 256: return launch(plain_batch_kernel<256, 4>, grid, block, a, pdl, s, smem);
+    case 32: return launch(plain_batch_kernel<32>, grid, block, a, pdl, s, smem);
+    case 64: return launch(plain_batch_kernel<64>, grid, block, a, pdl, s, smem);
+    case 128: return launch(plain_batch_kernel<128>, grid, block, a, pdl, s, smem);
+    case 256: return launch(plain_batch_kernel<256>, grid, block, a, pdl, s, smem);
     default: return cudaErrorInvalidValue;
   }
 }
