@@ -15,6 +15,7 @@
 
 #include "de_device.cuh"
 #include "de_internal.h"
+#include "de_pairs.cuh"
 
 namespace de {
 namespace {
@@ -23,41 +24,55 @@ using dev::Frag;
 using dev::kFull;
 
 constexpr uint64_t kAbsent64 = 0xC1E0000000000000ull;  // bits of (double)INT_MIN
-constexpr int kWarps = 8;
-
 int elementwise_grid(int64_t count) { return int(count / 256 + 1 < 152 * 8 ? count / 256 + 1 : 152 * 8); }
 
 // The attractive pass of every minibatch of one iteration in one launch (the
 // one-rank branch never merges its updates, so no row changes during the
-// iteration): one warp per work item, U neighbours in flight, split rows
-// combined in piece order.  Row i's update goes to Y[i] (FP32, from zero).  The
-// launch is hundreds of thousands of warps, so resident warps hide the gather's
-// latency: at dim 128 the kernel is held to 48 registers for five CTAs per SM.
-template <int D, int U>
-__global__ void __launch_bounds__(kWarps * 32, D == 128 ? 5 : 1) sparse_attract_kernel(const SpmmArgs a) {
+// iteration): one warp per work item, split rows combined in piece order.  Row i's
+// update goes to Y[i] (FP32, from zero).  The launch is hundreds of thousands of warps,
+// so resident warps hide the gather's latency, and the registers are held down for
+// them.  The sums keep the order of whole-warp rows at every dim (the collector adds
+// the updates up in 64 bits): from dim 128 on that is dev::pair_window's, below it is
+// dev::pair_forces'.  R-MAT of 131,072 vertices, dim 64 / 128 / 256: 187 / 231 / 610 us
+// an iteration -> 160 / 198 / 344 (four rows in flight; eight, or eight resident CTAs,
+// were slower at dim 128: 423 and 222).
+template <int D>
+constexpr int kAttractMinBlocks = D >= 256 ? 7 : D == 128 ? 12 : 8;
+
+template <int D>
+__global__ void __launch_bounds__(kPlainWarps * 32, kAttractMinBlocks<D>) sparse_attract_kernel(const SpmmArgs a) {
   const int lane = threadIdx.x & 31;
-  const int64_t gw = blockIdx.x * int64_t(kWarps) + (threadIdx.x >> 5);
+  const int64_t gw = blockIdx.x * int64_t(kPlainWarps) + (threadIdx.x >> 5);
   if (gw >= a.n_items) return;
   const WorkItem it = a.items[gw];
-  const int j = it.batch;
-  float *const P = a.P + size_t(__ldg(a.slot_off + j)) * D;
-  int32_t *const counters = a.counters + __ldg(a.counter_off + j);
-  const int64_t row = int64_t(j) * a.batch + it.row;
-  Frag<D> xi, acc;
-  dev::load_nc(xi, a.X + size_t(row) * D, lane);
-  acc.zero();
+  const int64_t row = int64_t(it.batch) * a.batch + it.row;
+  const float *const own = a.X + size_t(row) * D;
+  const int cnt = it.e_end - it.e_begin;  // at most 32
+  const int id = lane < cnt ? __ldg(a.col + it.e_begin + lane) : -1;
   float unused_loss = 0.f;
-  const int cnt = it.e_end - it.e_begin;
-  for (int k0 = 0; k0 < cnt; k0 += 32) {
-    const int ids = k0 + lane < cnt ? __ldg(a.col + it.e_begin + k0 + lane) : -1;
-    const int kn = min(32, cnt - k0);
-    for (int k = 0; k < kn; k += U) {
+  Frag<D> acc;
+  if constexpr (D >= 128) {
+    static_assert(dev::Lay<D>::LP == 32, "a whole warp holds a row");
+    const dev::PairCtx c(a.lr, a.bound, false);
+    dev::LaneRow<D> xi, sum;
+    dev::load_lanes<D, dev::kFinal>(xi, own, lane);
+    sum.zero();
+    dev::pair_window<D, dev::kFinal, 4>(sum, xi, id >= 0 ? a.X + size_t(id) * D : own, __ballot_sync(kFull, id >= 0), 0u,
+                                     c, unused_loss, lane);
+#pragma unroll
+    for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] = sum.v[t];
+  } else {
+    constexpr int U = 8;
+    Frag<D> xi;
+    dev::load_nc(xi, own, lane);
+    acc.zero();
+    for (int k = 0; k < cnt; k += U) {
       Frag<D> xn[U];
       unsigned valid = 0;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int nb = __shfl_sync(kFull, ids, (k + u) & 31);
-        if (k + u < kn) {
+        const int nb = __shfl_sync(kFull, id, (k + u) & 31);
+        if (k + u < cnt) {
           dev::load_nc(xn[u], a.X + size_t(nb) * D, lane);
           valid |= 1u << u;
         } else {
@@ -69,20 +84,9 @@ __global__ void __launch_bounds__(kWarps * 32, D == 128 ? 5 : 1) sparse_attract_
   }
   bool owner = true;
   if (it.nparts > 1) {
-    const int NP = it.nparts;
-    const int g = it.part / kCombineGroup;
-    const int ng = (NP + kCombineGroup - 1) / kCombineGroup;
-    const int gsize = min(kCombineGroup, NP - g * kCombineGroup);
+    float *const P = a.P + size_t(__ldg(a.slot_off + it.batch)) * D;
     dev::store<D, true>(acc, P + size_t(it.first_slot + it.part) * D, lane);
-    owner = dev::arrive_last(counters + it.counter + g, gsize, lane);
-    if (owner) {
-      dev::sum_slots(acc, P + size_t(it.first_slot + g * kCombineGroup) * D, gsize, lane);
-      if (ng > 1) {
-        dev::store<D, true>(acc, P + size_t(it.first_slot + NP + g) * D, lane);
-        owner = dev::arrive_last(counters + it.counter + ng, ng, lane);
-        if (owner) dev::sum_slots(acc, P + size_t(it.first_slot + NP) * D, ng, lane);
-      }
-    }
+    owner = dev::combine_parts<D>(acc, it, P, a.counters + __ldg(a.counter_off + it.batch), lane);
   }
   if (owner) dev::store<D, false>(acc, a.Y + size_t(row) * D, lane);
 }
@@ -181,21 +185,79 @@ __device__ __forceinline__ uint64_t order_key(double v) {
 __device__ __forceinline__ uint64_t order_key(float v) {
   uint32_t b = __float_as_uint(v);
   if (b == 0x80000000u) b = 0;
-  return (b >> 31) ? uint64_t(~b) : uint64_t(b | 0x80000000u);
+  return uint64_t((b >> 31) ? ~b : (b | 0x80000000u)) << 32;
 }
 
 // Top-k pruning (preserveHighestK, sparse_embedding.hpp:745-767): in every row
 // the dim - keep smallest values become absent; at equal values the lower dim
-// goes first.  One warp per row, lane l holding dims [lN, lN + N): a bitonic
-// sort of the row's (key, dim) pairs in registers (partners across lanes by
-// shuffle, within a lane directly), after which sorted position p < dim - keep
-// names a dim to drop.  When half the row is dropped (density 0.5) the first
-// step of the last merge already puts the D/2 smallest pairs below position
-// D/2, and the remaining steps, which only order the halves, are skipped.
+// goes first.  One warp per row, lane l holding dims [lN, lN + N).  The boundary
+// between the two sets is found bit by bit from the highest bit in which the row's
+// keys differ: a bit of the threshold is set when fewer than dim - keep keys lie
+// below it, and the search ends as soon as exactly that many do, which for distinct
+// values takes about as many bits as tell the two middle ones apart (a sorting
+// network takes its 22 to 28 stages over all keys; with the count before it, 131,072
+// rows at density 0.5: dim 128 289 -> 176 us, dim 256 922 -> 315 us).  Only when keys
+// are equal at the boundary does it come to the last bit, and the lowest of those dims are dropped.
 // T = double: the FP64 rows (absent = INT_MIN) and their mirror; T = float: the
 // mirror alone.  With `present` set the rows are pruned only when
 // floor(present / n) > keep (sparse_embedding.hpp:172-181), decided
 // here so that the host need not wait.
+template <int N, typename T>
+__device__ __forceinline__ void load_values(T (&v)[N], const T *p) {
+  constexpr int W = int(16 / sizeof(T)) < N ? int(16 / sizeof(T)) : N;  // values of a load
+  struct alignas(W * sizeof(T)) Pack { T x[W]; };
+#pragma unroll
+  for (int i = 0; i < N; i += W) {
+    const Pack t = *reinterpret_cast<const Pack *>(p + i);
+#pragma unroll
+    for (int k = 0; k < W; ++k) v[i + k] = t.x[k];
+  }
+}
+template <int N, typename T>
+__device__ __forceinline__ void store_values(T *p, const T (&v)[N]) {
+  constexpr int W = int(16 / sizeof(T)) < N ? int(16 / sizeof(T)) : N;
+  struct alignas(W * sizeof(T)) Pack { T x[W]; };
+#pragma unroll
+  for (int i = 0; i < N; i += W) {
+    Pack t;
+#pragma unroll
+    for (int k = 0; k < W; ++k) t.x[k] = v[i + k];
+    *reinterpret_cast<Pack *>(p + i) = t;
+  }
+}
+
+// The warp's words w[t] with in(t): the largest *bound with at most `want` of them
+// below it; returns how many lie below and stops early at exactly `want`.  Starts at
+// the highest bit, or with kAll (every word is in) at the highest in which they differ.
+template <int N, bool kAll, typename In>
+__device__ __forceinline__ int boundary(const uint32_t (&w)[N], int want, uint32_t *bound, In in) {
+  int bit = 31;
+  uint32_t b = 0;
+  if constexpr (kAll) {
+    const uint32_t first = __shfl_sync(kFull, w[0], 0);
+    uint32_t diff = 0;
+#pragma unroll
+    for (int t = 0; t < N; ++t) diff |= w[t] ^ first;
+    diff = __reduce_or_sync(kFull, diff);
+    bit = 31 - __clz(int(diff));  // -1: all the same
+    b = bit == 31 ? 0u : bit < 0 ? first : first & ~((2u << bit) - 1);
+  }
+  int below = 0;
+  for (; bit >= 0; --bit) {
+    const uint32_t cand = b | (1u << bit);
+    int c = 0;
+#pragma unroll
+    for (int t = 0; t < N; ++t) c += in(t) && w[t] < cand;
+    c = __reduce_add_sync(kFull, c);
+    if (c > want) continue;
+    b = cand;
+    below = c;
+    if (c == want) break;
+  }
+  *bound = b;
+  return below;
+}
+
 template <int D, typename T>
 __global__ void __launch_bounds__(256) sparse_prune_kernel(T *xs, float *x32, int64_t n, int32_t keep,
                                                            const unsigned long long *present) {
@@ -203,55 +265,61 @@ __global__ void __launch_bounds__(256) sparse_prune_kernel(T *xs, float *x32, in
   if (present && static_cast<int>(double(*present) / double(n)) <= keep) return;
   const int lane = threadIdx.x & 31;
   const int nullify = D - keep;
+  if (nullify <= 0) return;
   for (int64_t row = blockIdx.x * int64_t(blockDim.x >> 5) + (threadIdx.x >> 5); row < n;
        row += int64_t(gridDim.x) * (blockDim.x >> 5)) {
-    T *xr = xs + row * D;
+    T *xr = xs + row * D + lane * N;
+    T val[N];
+    load_values<N>(val, xr);
     uint64_t key[N];
-    int idx[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) key[t] = order_key(val[t]);
+    // keys below `bound` are dropped, and the first `ties` of those equal to it: the
+    // high words first, the low ones only among keys equal in the high word
+    uint64_t bound = ~uint64_t(0);
+    int ties = D;
+    if (nullify < D) {
+      uint32_t hi[N];
+#pragma unroll
+      for (int t = 0; t < N; ++t) hi[t] = uint32_t(key[t] >> 32);
+      int want = nullify;
+      uint32_t bhi = 0, blo = 0;
+      want -= boundary<N, true>(hi, want, &bhi, [](int) { return true; });
+      if (want > 0) {
+        uint32_t lo[N];
+#pragma unroll
+        for (int t = 0; t < N; ++t) lo[t] = uint32_t(key[t]);
+        want -= boundary<N, false>(lo, want, &blo, [&](int t) { return hi[t] == bhi; });
+      }
+      bound = (uint64_t(bhi) << 32) | blo;
+      ties = want;
+    }
+    int rank = 0;  // keys equal to `bound` in lower dims
+    if (ties > 0) {
+      int own = 0;
+#pragma unroll
+      for (int t = 0; t < N; ++t) own += key[t] == bound;
+      rank = own;
+#pragma unroll
+      for (int m = 1; m < 32; m <<= 1) {
+        const int up = __shfl_up_sync(kFull, rank, m);
+        if (lane >= m) rank += up;
+      }
+      rank -= own;
+    }
+    float mirror[N];
 #pragma unroll
     for (int t = 0; t < N; ++t) {
-      idx[t] = lane * N + t;
-      key[t] = order_key(xr[idx[t]]);
-    }
-#pragma unroll
-    for (int k = 2; k <= D; k <<= 1) {
-#pragma unroll
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        uint64_t pk[N];
-        int pi[N];
-#pragma unroll
-        for (int t = 0; t < N; ++t) {
-          if (j >= N) {
-            pk[t] = __shfl_xor_sync(kFull, key[t], j / N);
-            pi[t] = __shfl_xor_sync(kFull, idx[t], j / N);
-          } else {
-            pk[t] = key[t ^ j];
-            pi[t] = idx[t ^ j];
-          }
-        }
-#pragma unroll
-        for (int t = 0; t < N; ++t) {
-          const int i = lane * N + t;
-          const bool keep_min = ((i & j) == 0) == ((i & k) == 0);
-          const bool p_less = pk[t] < key[t] || (pk[t] == key[t] && pi[t] < idx[t]);
-          if (keep_min == p_less) {
-            key[t] = pk[t];
-            idx[t] = pi[t];
-          }
-        }
-        if (k == D && j == D / 2 && nullify == D / 2) break;
+      const bool drop = key[t] < bound || (key[t] == bound && rank++ < ties);
+      if constexpr (sizeof(T) == 8) {
+        mirror[t] = drop || __double_as_longlong(val[t]) == int64_t(kAbsent64) ? 0.f : float(val[t]);
+        if (drop) val[t] = __longlong_as_double(int64_t(kAbsent64));
+      } else if (drop) {
+        val[t] = 0.f;  // xs is the mirror itself
       }
     }
-#pragma unroll
-    for (int t = 0; t < N; ++t)
-      if (lane * N + t < nullify) {
-        if constexpr (sizeof(T) == 8) {
-          xr[idx[t]] = __longlong_as_double(int64_t(kAbsent64));
-          x32[row * D + idx[t]] = 0.f;
-        } else {
-          xr[idx[t]] = 0.f;  // xs is the mirror itself
-        }
-      }
+    store_values<N>(xr, val);
+    if constexpr (sizeof(T) == 8) store_values<N>(x32 + row * D + lane * N, mirror);
   }
 }
 
@@ -287,14 +355,14 @@ cudaError_t prune_dispatch(int dim, T *xs, float *x32, int64_t n, int32_t keep, 
 }  // namespace
 
 cudaError_t launch_sparse_attract(int dim, const SpmmArgs &a, cudaStream_t s) {
-  const int64_t grid = (a.n_items + kWarps - 1) / kWarps;
+  const int64_t grid = (a.n_items + kPlainWarps - 1) / kPlainWarps;
   if (grid == 0) return cudaSuccess;
   if (grid >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
   switch (dim) {
-    case 32: sparse_attract_kernel<32, 8><<<unsigned(grid), kWarps * 32, 0, s>>>(a); break;
-    case 64: sparse_attract_kernel<64, 8><<<unsigned(grid), kWarps * 32, 0, s>>>(a); break;
-    case 128: sparse_attract_kernel<128, 4><<<unsigned(grid), kWarps * 32, 0, s>>>(a); break;
-    case 256: sparse_attract_kernel<256, 2><<<unsigned(grid), kWarps * 32, 0, s>>>(a); break;
+    case 32: sparse_attract_kernel<32><<<unsigned(grid), kPlainWarps * 32, 0, s>>>(a); break;
+    case 64: sparse_attract_kernel<64><<<unsigned(grid), kPlainWarps * 32, 0, s>>>(a); break;
+    case 128: sparse_attract_kernel<128><<<unsigned(grid), kPlainWarps * 32, 0, s>>>(a); break;
+    case 256: sparse_attract_kernel<256><<<unsigned(grid), kPlainWarps * 32, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
