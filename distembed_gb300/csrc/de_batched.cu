@@ -197,9 +197,32 @@ int bgrow(de_batch *b, T **p, size_t *cap, size_t need) {
   return DE_OK;
 }
 
+// items[first, end) by falling length, equal lengths in their present order: lengths
+// are at most `cap`, so a counting sort, where the counters are not more than the items.
+void order_items(std::vector<WorkItem> &items, size_t first, int cap, std::vector<WorkItem> &spare,
+                 std::vector<size_t> &place) {
+  auto length = [](const WorkItem &w) { return w.e_end - w.e_begin; };
+  if (size_t(cap) > items.size() - first) {
+    std::stable_sort(items.begin() + first, items.end(),
+                     [&](const WorkItem &x, const WorkItem &y) { return length(x) > length(y); });
+    return;
+  }
+  place.assign(size_t(cap) + 1, 0);
+  for (size_t i = first; i < items.size(); ++i) ++place[length(items[i])];
+  size_t next = first;
+  for (int l = cap; l >= 0; --l) {
+    const size_t c = place[l];
+    place[l] = next;
+    next += c;
+  }
+  spare.assign(items.begin() + first, items.end());
+  for (const WorkItem &w : spare) items[place[length(w)]++] = w;
+}
+
 // Work items and split rows of every minibatch of every graph (edge cap `cap`).
 int build_batched_schedule(de_batch *b, int B, int cap) {
-  std::vector<WorkItem> items;
+  std::vector<WorkItem> items, spare;
+  std::vector<size_t> place;
   std::vector<int64_t> bitem{0};
   std::vector<int32_t> bsplit{0};
   std::vector<SplitRow> splits;
@@ -237,9 +260,7 @@ int build_batched_schedule(de_batch *b, int B, int cap) {
           slot += np;
         }
       }
-      std::stable_sort(items.begin() + first, items.end(), [](const WorkItem &x, const WorkItem &y) {
-        return (x.e_end - x.e_begin) > (y.e_end - y.e_begin);
-      });
+      order_items(items, first, cap, spare, place);
       max_slots = std::max(max_slots, slot);
       bitem.push_back(int64_t(items.size()));
       max_items = std::max<int64_t>(max_items, bitem.back() - bitem[bitem.size() - 2]);

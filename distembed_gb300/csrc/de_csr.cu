@@ -86,6 +86,25 @@ __global__ void coo_keys_kernel(const int64_t *__restrict__ row, const int64_t *
   }
 }
 
+// dst = src as int32; counters[0] counts the columns outside [0, n), counters[1] those
+// equal to n - 1.
+__global__ void __launch_bounds__(256) check_columns_kernel(const int64_t *__restrict__ src, int32_t *__restrict__ dst,
+                                                            int64_t count, int64_t n, unsigned long long *counters) {
+  unsigned bad = 0, last = 0;
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t c = src[i];
+    dst[i] = int32_t(c);
+    bad += c < 0 || c >= n;
+    last += c == n - 1;
+  }
+  bad = __reduce_add_sync(0xffffffffu, bad);
+  last = __reduce_add_sync(0xffffffffu, last);
+  if ((threadIdx.x & 31) == 0) {
+    if (bad) atomicAdd(counters, static_cast<unsigned long long>(bad));
+    if (last) atomicAdd(counters + 1, static_cast<unsigned long long>(last));
+  }
+}
+
 int grid_for(int64_t n) { return int(std::min<int64_t>((n + 255) / 256 + 1, 152 * 16)); }
 
 struct DeviceBuffers {
@@ -204,6 +223,14 @@ void touch_pages(void *p, size_t bytes) {
 }
 
 }  // namespace
+
+cudaError_t launch_columns(const int64_t *src, int32_t *dst, int64_t count, int64_t n, unsigned long long *counters,
+                           cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  check_columns_kernel<<<grid_for(count), 256, 0, s>>>(src, dst, count, n, counters);
+  return cudaGetLastError();
+}
+
 }  // namespace de
 
 extern "C" {

@@ -213,6 +213,11 @@ int create_handle(int64_t n, const int64_t *rowptr, const int64_t *col, int64_t 
 // the handle's stream.
 int copy_loss(de_handle *h, double *out, int32_t epochs);
 
+// CSR columns to int32 (de_csr.cu): counters[0] += columns outside [0, n), counters[1] +=
+// columns equal to n - 1.
+cudaError_t launch_columns(const int64_t *src, int32_t *dst, int64_t count, int64_t n, unsigned long long *counters,
+                           cudaStream_t s);
+
 // Launchers (de_plain.cu).  pdl: launch with a programmatic dependency on the
 // previous kernel in the stream.
 // teams: several warps to a work item where plain_team_warps says so (one otherwise).
