@@ -30,6 +30,7 @@
 #include "de_async.cuh"
 #include "de_device.cuh"
 #include "de_internal.h"
+#include "de_pairs.cuh"
 
 namespace de {
 namespace {
@@ -84,90 +85,7 @@ __device__ __forceinline__ void load_bf16_row(Frag<D> &f, const __nv_bfloat16 *r
   }
 }
 
-template <int D>
-__device__ __forceinline__ void store_f32_contig(const Frag<D> &f, float *row, int lane) {
-  constexpr int N = D / 32;
-  float *p = row + lane * N;
-  if constexpr (N % 4 == 0) {
-#pragma unroll
-    for (int i = 0; i < N; i += 4) *reinterpret_cast<float4 *>(p + i) = make_float4(f.v[i], f.v[i + 1], f.v[i + 2], f.v[i + 3]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < N; i += 2) *reinterpret_cast<float2 *>(p + i) = make_float2(f.v[i], f.v[i + 1]);
-  }
-}
-
 // ------------------------------------------------------------ attractive + gather
-
-// A lane's D/32 BF16 components of a row as loaded (16, 8 or 4 bytes), unpacked
-// to FP32 only when used, so that rows in flight cost half the registers.
-template <int D>
-struct RawRow {
-  static constexpr int W = D / 64;  // 32-bit words per lane
-  uint32_t w[W];
-};
-
-template <int D>
-__device__ __forceinline__ void load_raw(RawRow<D> &r, const __nv_bfloat16 *row, int lane) {
-  constexpr int W = RawRow<D>::W;
-  const __nv_bfloat16 *p = row + lane * (D / 32);
-  if constexpr (W == 4) {
-    const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p));
-    r.w[0] = u.x, r.w[1] = u.y, r.w[2] = u.z, r.w[3] = u.w;
-  } else if constexpr (W == 2) {
-    const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
-    r.w[0] = u.x, r.w[1] = u.y;
-  } else {
-    static_assert(W == 1, "dim 64, 128 or 256");
-    r.w[0] = __ldg(reinterpret_cast<const unsigned *>(p));
-  }
-}
-
-// The same values load_bf16_row produces.
-template <int D>
-__device__ __forceinline__ void unpack_row(Frag<D> &f, const RawRow<D> &r) {
-#pragma unroll
-  for (int i = 0; i < RawRow<D>::W; ++i) {
-    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&r.w[i]));
-    f.v[2 * i] = t.x;
-    f.v[2 * i + 1] = t.y;
-  }
-}
-
-// The rows of CSR entries k .. k+U-1 (lane j of `ids`: the column of entry j,
-// -1 for none) as raw BF16; bit u of the result: entry k+u is a row.
-template <int D, int U>
-__device__ __forceinline__ unsigned fetch_group(const BF16BatchArgs &a, RawRow<D> (&raw)[U], int ids, int k, int lane) {
-  unsigned mask = 0;
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int n = __shfl_sync(kFull, ids, k + u);
-    if (n >= 0) {
-      load_raw<D>(raw[u], a.xb + size_t(n) * D, lane);
-      mask |= 1u << u;
-    }
-  }
-  return mask;
-}
-
-template <int D, int U>
-__device__ __forceinline__ void bf16_force_group(const BF16BatchArgs &a, Frag<D> &acc, const Frag<D> &xi, int ids,
-                                                 int k, float lr, float bound, bool want_loss, float &loss,
-                                                 int lane) {
-  Frag<D> xn[U];
-  unsigned mask = 0;
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int n = __shfl_sync(kFull, ids, k + u);
-    if (n >= 0) {
-      load_bf16_row(xn[u], a.xb + size_t(n) * D, lane);
-      mask |= 1u << u;
-    } else {
-      xn[u] = xi;
-    }
-  }
-  if (mask) pair_forces<D, U, true>(acc, xi, xn, mask, lr, bound, want_loss, loss, lane);
-}
 
 // The minibatch's negatives gathered once: N (k x dim, zero rows for padding),
 // |n|^2 and ids.  A CTA takes 32 consecutive negatives, one warp each: the warp
@@ -219,76 +137,47 @@ __global__ void __launch_bounds__(kGatherTile * 32) bf16_gather_kernel(const BF1
   }
 }
 
-template <int D, int U>
-__global__ void __launch_bounds__(kPlainWarps * 32, 6) bf16_attract_kernel(const BF16BatchArgs a) {
+// The attractive pass, a warp per work item, pairs as in the FP32 kernels (dev::
+// pair_window) on the BF16 rows: 16 bytes of a row per lane, so below dim 256 a warp
+// takes several pairs a step.  Resident warps count for more than a few spilled words.
+// R-MAT, B = 4096 to 16384, us a launch: dim 256 39.5 -> 32.6 (two steps in flight 39.1),
+// dim 128 27.5 -> 23.3, dim 64 30.4 -> 23.3.
+template <int D, bool kLoss>
+__global__ void __launch_bounds__(kPlainWarps * 32, D == 256 ? 8 : 10) bf16_attract_kernel(const BF16BatchArgs a) {
+  typedef B16Rows<D, D == 256 ? 4 : 2> R;
   const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  const bool want_loss = a.compute_loss != 0;
-  const int epoch = a.epoch[0];
-  const float lr = a.lr[epoch];
-
-  const int gw = blockIdx.x * kPlainWarps + wib;
+  const int gw = blockIdx.x * kPlainWarps + (threadIdx.x >> 5);
   if (gw >= a.n_items) return;
   const WorkItem it = a.items[gw];
+  const int epoch = a.epoch[0];
+  const PairCtx c(a.lr[epoch], a.bound, kLoss);
   const int skip = a.quirks ? a.n - 1 : -1;  // edges into n-1 are dropped (algo.hpp:399-405, 538)
-  const int cnt = it.e_end - it.e_begin;
+  const int cnt = it.e_end - it.e_begin;     // at most 32
   if (cnt == 0) {  // a row without CSR entries: no attractive update (the update kernel reads none)
-    if (want_loss && lane == 0) a.loss_item[a.loss_off + gw] = 0.0;
+    if (kLoss && lane == 0) a.loss_item[a.loss_off + gw] = 0.0;
     return;
   }
-  int ids = -1;
-  if (lane < cnt) {
-    ids = __ldg(a.col + it.e_begin + lane);
-    if (ids == skip) ids = -1;
-  }
-  Frag<D> xi, acc;
-  load_bf16_row(xi, a.xb + size_t(a.base + it.row) * D, lane);
+  const __nv_bfloat16 *const own = a.xb + size_t(a.base + it.row) * D;
+  const int id = lane < cnt ? __ldg(a.col + it.e_begin + lane) : skip;
+  const bool counts = lane < cnt && id != skip;
+  uint4 raw;
+  R::load(raw, own, lane % R::LP);
+  const LaneVec<8> xi = R::unpack(raw);
+  LaneVec<8> acc;
   acc.zero();
   float loss = 0.f;  // this item's loss terms (FP32); the epoch sum is FP64
-  // groups of U, software-pipelined: the next group's rows are in flight (as
-  // raw BF16) while this group's forces are computed; a last group of at most
-  // U/2 entries runs as a group of U/2
-  int k = 0;
-  if (U / 2 < cnt) {
-    RawRow<D> cur[U];
-    unsigned mcur = fetch_group<D, U>(a, cur, ids, 0, lane);
-    for (; k + U / 2 < cnt; k += U) {
-      RawRow<D> nxt[U];
-      unsigned mnxt = 0;
-      if (k + U + U / 2 < cnt) mnxt = fetch_group<D, U>(a, nxt, ids, k + U, lane);
-      Frag<D> xn[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if ((mcur >> u) & 1u) unpack_row<D>(xn[u], cur[u]);
-        else xn[u] = xi;
-      }
-      if (mcur) pair_forces<D, U, true>(acc, xi, xn, mcur, lr, a.bound, want_loss, loss, lane);
-#pragma unroll
-      for (int u = 0; u < U; ++u) cur[u] = nxt[u];
-      mcur = mnxt;
-    }
+  pair_window<R>(acc, xi, counts ? a.xb + size_t(id) * D : own, __ballot_sync(kFull, counts), 0u, c, loss, lane);
+  sum_lane_groups<R::LP>(acc);
+  // lanes [0, LP) hold the row, 8 components each
+  float *const out = a.abuf + size_t(it.row) * D;
+  float *const mine = it.nparts > 1 ? a.P + size_t(it.first_slot + it.part) * D : out;
+  if (lane < R::LP) {
+    __stcg(reinterpret_cast<float4 *>(mine) + 2 * lane, make_float4(acc.v[0], acc.v[1], acc.v[2], acc.v[3]));
+    __stcg(reinterpret_cast<float4 *>(mine) + 2 * lane + 1, make_float4(acc.v[4], acc.v[5], acc.v[6], acc.v[7]));
   }
-  if (k < cnt) bf16_force_group<D, U / 2>(a, acc, xi, ids, k, lr, a.bound, want_loss, loss, lane);
-
-  bool owner = true;
-  if (it.nparts > 1) {
-    const int P = it.nparts;
-    const int g = it.part / kCombineGroup;
-    const int ng = (P + kCombineGroup - 1) / kCombineGroup;
-    const int gsize = min(kCombineGroup, P - g * kCombineGroup);
-    store<D, true>(acc, a.P + size_t(it.first_slot + it.part) * D, lane);
-    owner = arrive_last(a.counters + it.counter + g, gsize, lane);
-    if (owner) {
-      sum_slots(acc, a.P + size_t(it.first_slot + g * kCombineGroup) * D, gsize, lane);
-      if (ng > 1) {
-        store<D, true>(acc, a.P + size_t(it.first_slot + P + g) * D, lane);
-        owner = arrive_last(a.counters + it.counter + ng, ng, lane);
-        if (owner) sum_slots(acc, a.P + size_t(it.first_slot + P) * D, ng, lane);
-      }
-    }
-  }
-  if (owner) store_f32_contig(acc, a.abuf + size_t(it.row) * D, lane);
-  if (want_loss) {
+  Frag<D> sum;
+  if (it.nparts > 1 && combine_parts<D>(sum, it, a.P, a.counters, lane)) store<D, false>(sum, out, lane);
+  if (kLoss) {
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) loss += __shfl_xor_sync(kFull, loss, m);
     if (lane == 0) a.loss_item[a.loss_off + gw] = double(loss);
@@ -384,7 +273,7 @@ struct RepulseSmem {
   static constexpr int kX = kAtoms * kTileRows * 128;    // X tile
   static constexpr int kN = kAtoms * kChunk * 128;       // one chunk of N (B operand of both GEMMs)
   static_assert(kX == 2 * kN, "the X tile takes two stages");
-  static constexpr int kMisc = 16384;                    // per-row exchanges, flags and losses
+  static constexpr int kMisc = 4096;                     // per-row exchanges between the column halves
   static constexpr int offN = 0;
   static constexpr int offX = offN + (kStages - 2) * kN;  // first over the last two stages
   static constexpr int offMisc = offN + kStages * kN;
@@ -406,29 +295,14 @@ struct RepulseSmem {
 // through a ring of six stages, the last two of which first hold the TMA copy
 // of the X tile (until it is in tensor memory).
 //
-// KS = 2: the negatives of a tile are split between the two CTAs of a cluster
-// (rank 0: the first ceil(chunks / 2) chunks, rank 1 the rest), so twice as
-// many SMs work on a minibatch.  Rank r owns tile rows [64 r, 64 r + 64).  Each
-// CTA stages its partial force (its row sums) x - (its F) of all 128 rows in its
-// shared memory; once the peer has signalled (a release arrive on this CTA's
-// PEER_FREE barrier) that its incoming area is free, one warp pushes the peer's
-// 64 rows, their flags and losses with bulk copies into the peer's shared memory,
-// completing on the peer's INCOMING barrier; each CTA then adds the two partials
-// of its rows and stores them, and waits (PEER_GOT) until the peer has received
-// its rows before its shared memory ends.  Partial sums are combined as own +
-// peer, the same value on either rank.  Every wait is bounded.
+// The negatives of a tile are split between `ksplit` CTAs (bf16_ksplit), so that more
+// SMs work on a minibatch: each stores its partial force (its row sums) x - (its F) in
+// its own part of rbuf, and the update kernel adds the parts in order.  (Two CTAs as a
+// cluster that exchanged half their rows and stored the sums took 25.2 us a launch
+// against 22.5, 8,192 rows, 1,024 negatives, dim 256.)  Every wait is bounded.
 constexpr int kEpiThreads = 256;
 constexpr int kRepulseThreads = kEpiThreads + 64;
 
-__device__ __forceinline__ int cta_rank_in_cluster() {
-  int r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// Release arrive on a barrier of the peer CTA (address from peer_addr).
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 // mbar_wait for threads that may wait long and share their SM sub-partition
 // with the MMA-issuing thread: each poll may suspend the thread (up to 2 us,
 // woken early when the phase completes) instead of spinning on the issue slots;
@@ -448,36 +322,7 @@ __device__ __forceinline__ bool mbar_wait_sleep(uint32_t bar, uint32_t parity, i
   *reinterpret_cast<volatile int *>(err_shared) = 1;
   return false;
 }
-// mbar_wait with cluster-scope acquire (the phase was completed by the peer CTA).
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int *err_shared) {
-  for (long it = 0; it < kSpinLimit; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (*reinterpret_cast<volatile int *>(err_shared)) return false;
-  }
-  *reinterpret_cast<volatile int *>(err_shared) = 1;
-  return false;
-}
-__device__ __forceinline__ uint32_t peer_addr(uint32_t local, int peer) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(peer));
-  return r;
-}
-// Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from
-// this CTA's shared memory into the peer CTA's (dst, bar: peer_addr addresses),
-// completing on the peer's barrier.
-__device__ __forceinline__ void bulk_s2peer(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "r"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
-template <int D, int KS>
+template <int D>
 __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                const __grid_constant__ CUtensorMap map_n,
                                                                const BF16BatchArgs a) {
@@ -490,22 +335,19 @@ __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const 
   __shared__ float2 negmeta[2][kChunk];  // (|n|^2, vertex id) of a chunk's negatives
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunks = a.kpad / kChunk;
-  const int ks = KS == 2 ? cta_rank_in_cluster() : 0;
-  const int peer = ks ^ 1;  // KS = 2: the other CTA of the cluster
-  const int tile_base = (blockIdx.x / KS) * kTileRows;  // row offset within the minibatch
-  // this CTA's chunks [c_begin, c_end) (KS = 2 needs at least two chunks)
-  const int c_begin = ks == 0 ? 0 : (nchunks + 1) / 2;
-  const int c_end = (KS == 1 || ks == 1) ? nchunks : (nchunks + 1) / 2;
-  const int nloc = c_end - c_begin;
+  const int ks = blockIdx.x % a.ksplit;
+  const int tile_base = (blockIdx.x / a.ksplit) * kTileRows;  // row offset within the minibatch
+  // this CTA's chunks (ksplit is at most the number of chunks)
+  const int c_begin = nchunks * ks / a.ksplit;
+  const int nloc = nchunks * (ks + 1) / a.ksplit - c_begin;
 
   // barrier ids
   constexpr int NST = L::kStages;
   const uint32_t b0 = smem_u32(&bar[0]);
   auto B = [&](int i) { return b0 + 8u * uint32_t(i); };
   const int FULL_X = 0, FULL_N = 1, FREE_N = FULL_N + NST, X_TMEM = FREE_N + NST, S_FULL = X_TMEM + 1,
-            C_FULL = S_FULL + 2, F_DONE = C_FULL + 2, INCOMING = F_DONE + 1, PEER_FREE = INCOMING + 1,
-            PEER_GOT = PEER_FREE + 1;
-  static_assert(1 + 2 * NST + 1 + 4 + 4 <= 24, "barrier slots");
+            C_FULL = S_FULL + 2, F_DONE = C_FULL + 2;
+  static_assert(1 + 2 * NST + 1 + 4 + 1 <= 24, "barrier slots");
   constexpr uint32_t kColX = 128, kColF = 256;  // tensor-memory columns of X and F
   auto failed = [&]() { return *reinterpret_cast<volatile int *>(&err) != 0; };
 
@@ -522,9 +364,6 @@ __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const 
       mbar_init(B(C_FULL + i), kEpiThreads);
     }
     mbar_init(B(F_DONE), 1);
-    mbar_init(B(INCOMING), 1);
-    mbar_init(B(PEER_FREE), 1);
-    mbar_init(B(PEER_GOT), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 9) {
@@ -536,35 +375,18 @@ __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // KS = 2: every thread arrives once here, after the barrier initialisation,
-  // and waits once before this CTA first touches the peer's shared memory
-  if constexpr (KS == 2) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const uint32_t tmem = tmem_holder;
   const uint32_t sX = smem_u32(sm + L::offX);
   auto sN = [&](int st) { return smem_u32(sm + L::offN + st * L::kN); };
-  // the misc area: per-row exchanges between the two column halves ([0, 4096),
-  // used before the staging), then per tile row a flag (nonzero: the row's
-  // force is final) and, with KS = 2, its loss, then the peer's flags and losses
+  // the misc area: per-row exchanges between the two column halves
   unsigned char *const misc = sm + L::offMisc;
   float *const xx_part = reinterpret_cast<float *>(misc);
   float *const rs_part = reinterpret_cast<float *>(misc + 1024);
   double *const loss_part = reinterpret_cast<double *>(misc + 2048);
-  int *const row_flags = reinterpret_cast<int *>(misc + 4096);
-  double *const row_loss = reinterpret_cast<double *>(misc + 5120);
-  int *const in_flags = reinterpret_cast<int *>(misc + 8192);
-  double *const in_loss = reinterpret_cast<double *>(misc + 8448);
-  // after the GEMMs: the staged force rows (pitch D + 4 floats) over the N
-  // stages; KS = 2: after them the peer's partials of this CTA's 64 rows (the
-  // same pitch: one contiguous block, reaching into the then dead half-row
-  // exchange area of misc, before the row flags), their 64 flags and 64 losses
-  // in the misc area
+  // after the GEMMs: the staged force rows (pitch D + 4 floats) over the N stages
   constexpr int kPitch = D + 4;
-  constexpr int kStageBytes = kTileRows * kPitch * 4;
-  constexpr uint32_t kHalfRowsBytes = 64 * kPitch * 4;
   float *const stage = reinterpret_cast<float *>(sm + L::offN);
-  float *const in_rows = reinterpret_cast<float *>(sm + L::offN + kStageBytes);
-  static_assert(kStageBytes + kHalfRowsBytes <= L::offMisc - L::offN + 4096, "incoming rows end before the row flags");
-  constexpr uint32_t kInBytes = kHalfRowsBytes + 64 * 4 + 64 * 8;
+  static_assert(kTileRows * kPitch * 4 <= L::offMisc - L::offN, "the staged rows end before the misc area");
 
   if (warp == 8) {
     // ---------------- TMA producer
@@ -651,7 +473,6 @@ __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const 
     const int row_local = tile_base + t;
     const bool row_valid = row_local < a.rows;
     const bool rep_active = row_valid && row_local < rep_rows;
-    const int row_global = a.base + row_local;
     const float lr = a.lr[epoch];
     auto epi_sync = []() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
 
@@ -803,8 +624,7 @@ __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const 
     epi_sync();
     rowsum = rs_part[t] + rs_part[kTileRows + t];
     loss = loss_part[t] + loss_part[kTileRows + t];
-    if (KS == 1 && hf == 0 && row_valid && done) a.loss_row[row_global] = loss;
-    epi_sync();  // the staging below may overwrite the combine area
+    if (a.compute_loss && hf == 0 && row_valid && done) a.rloss[size_t(ks) * a.rstride + row_local] = loss;
 
     // Repulsive force rowsum * x - F of every tile row, staged as FP32 rows; x
     // comes from the BF16 X tile in tensor memory.  Thread (row t, half hf)
@@ -825,80 +645,21 @@ __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const 
                         rowsum * x1.x - __uint_as_float(f[d + 2]), rowsum * x1.y - __uint_as_float(f[d + 3]));
       }
     }
-    if (hf == 0) {
-      row_flags[t] = (row_valid && done) ? 1 : 0;
-      if (KS == 2) row_loss[t] = loss;
-    }
-    if constexpr (KS == 2) {
-      // the staged rows are read next by the bulk copy engine (async proxy)
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      epi_sync();
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-      if (tid == 0) {
-        // this CTA's incoming area is free and its INCOMING barrier expects the rows:
-        // tell the peer (a release arrive on the peer's PEER_FREE barrier)
-        mbar_expect_tx(B(INCOMING), kInBytes);
-        mbar_arrive_remote(peer_addr(B(PEER_FREE), peer));
-      }
-      // warp 0 pushes the partials of the peer's 64 rows (one contiguous block
-      // of staged rows), their flags and losses into the peer's shared memory
-      // once the peer has staged its own rows, completing on the peer's
-      // INCOMING barrier
-      if (warp == 0 && __all_sync(kFull, mbar_wait_cluster(B(PEER_FREE), 0, &err))) {
-        const int pr0 = peer * 64;
-        const uint32_t pbar = peer_addr(B(INCOMING), peer);
-        if (lane == 0) {
-          bulk_s2peer(peer_addr(smem_u32(in_rows), peer), smem_u32(stage + pr0 * kPitch), kHalfRowsBytes, pbar);
-          bulk_s2peer(peer_addr(smem_u32(in_flags), peer), smem_u32(&row_flags[pr0]), 64 * 4, pbar);
-          bulk_s2peer(peer_addr(smem_u32(in_loss), peer), smem_u32(&row_loss[pr0]), 64 * 8, pbar);
-        }
-      }
-    } else {
-      epi_sync();
-    }
-
+    epi_sync();
     // Coalesced store of lr * force, one warp per row, lane l the 16-byte
     // vectors l, l + 32, ... (every store instruction writes whole 32-byte
-    // sectors), into rbuf; bf16_apply_kernel adds it to the row together with
-    // the attractive update (which runs concurrently into abuf).
-    for (int rr = warp; KS == 1 && rr < kTileRows; rr += kEpiThreads / 32) {
-      if (row_flags[rr] == 0) continue;
+    // sectors), into this CTA's part of rbuf; bf16_apply_kernel adds the parts to the
+    // row together with the attractive update (which runs concurrently into abuf).
+    const int rows = min(kTileRows, a.rows - tile_base);
+    for (int rr = warp; done && rr < rows; rr += kEpiThreads / 32) {
       const float4 *src = reinterpret_cast<const float4 *>(stage + rr * kPitch);
-      float4 *rbp = reinterpret_cast<float4 *>(a.rbuf + size_t(tile_base + rr) * D);
+      float4 *rbp = reinterpret_cast<float4 *>(a.rbuf + (size_t(ks) * a.rstride + tile_base + rr) * D);
 #pragma unroll
       for (int v = lane; v < D / 4; v += 32) {
         const float4 f = src[v];
         rbp[v] = make_float4(lr * f.x, lr * f.y, lr * f.z, lr * f.w);
       }
     }
-    if constexpr (KS == 2) {
-      // this CTA's rows [64 ks, 64 ks + 64): own partial + the peer's
-      const bool in_ok = __all_sync(kFull, mbar_wait_cluster(B(INCOMING), 0, &err));
-      // the peer's copies into this CTA have landed, so the peer's staged rows
-      // are no longer read: tell the peer at once
-      if (tid == 0 && in_ok) mbar_arrive_remote(peer_addr(B(PEER_GOT), peer));
-      const int r0 = ks * 64;
-      for (int i = warp; in_ok && i < 64; i += kEpiThreads / 32) {
-        if (row_flags[r0 + i] == 0 || in_flags[i] == 0) continue;
-        const float4 *own = reinterpret_cast<const float4 *>(stage + (r0 + i) * kPitch);
-        const float4 *oth = reinterpret_cast<const float4 *>(in_rows + i * kPitch);
-        float4 *rbp = reinterpret_cast<float4 *>(a.rbuf + size_t(tile_base + r0 + i) * D);
-#pragma unroll
-        for (int v = lane; v < D / 4; v += 32) {
-          const float4 p = own[v], q = oth[v];
-          rbp[v] = make_float4(lr * (p.x + q.x), lr * (p.y + q.y), lr * (p.z + q.z), lr * (p.w + q.w));
-        }
-      }
-      if (in_ok && tid < 64 && row_flags[r0 + tid] != 0 && in_flags[tid] != 0)
-        a.loss_row[a.base + tile_base + r0 + tid] = row_loss[r0 + tid] + in_loss[tid];
-      // the CTA (and its shared memory) ends only after the peer has received
-      // this CTA's rows
-      if (tid == 0) mbar_wait_cluster(B(PEER_GOT), 0, &err);
-    }
-  }
-  if constexpr (KS == 2) {
-    __syncwarp();
-    if (warp >= kEpiThreads / 32) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -943,7 +704,8 @@ __device__ __forceinline__ void st_contig(float *p, const float (&v)[N]) {
 }
 
 // One warp per row of the minibatch: x += abuf + rbuf (attractive and GEMM
-// repulsive updates, algo.hpp:651-666), plus, for a row with exact-path pairs
+// repulsive updates, the latter the sum of the tile's CTAs in order, algo.hpp:651-666),
+// plus, for a row with exact-path pairs
 // (bitmask bits), those pairs added in FP32 on the BF16 values with the
 // per-component clip (algo.hpp:633-645), in negative order; the bits are cleared.
 template <int D>
@@ -967,6 +729,15 @@ __global__ void __launch_bounds__(256) bf16_apply_kernel(const BF16BatchArgs a) 
     ld_contig<N>(mv, xm);
     ld_contig<N>(av, a.abuf + size_t(row_local) * D + lane * N);
     ld_contig<N>(rv, a.rbuf + size_t(row_local) * D + lane * N);
+    for (int k = 1; k < a.ksplit; ++k) {
+      float more[N];
+      ld_contig<N>(more, a.rbuf + (size_t(k) * a.rstride + row_local) * D + lane * N);
+#pragma unroll
+      for (int t = 0; t < N; ++t) rv[t] += more[t];
+    }
+    double row_loss = 0.0;
+    if (a.compute_loss && lane == 0)
+      for (int k = 0; k < a.ksplit; ++k) row_loss += a.rloss[size_t(k) * a.rstride + row_local];
     Frag<D> acc;
     acc.zero();
     const bool exact = __any_sync(kFull, my_word != 0u);
@@ -998,8 +769,9 @@ __global__ void __launch_bounds__(256) bf16_apply_kernel(const BF16BatchArgs a) 
         }
       }
       if (lane < kNearWords) bits_row[lane] = 0u;
-      if (lane == 0) a.loss_row[row] += double(loss);
+      row_loss += double(loss);
     }
+    if (a.compute_loss && lane == 0) a.loss_row[row] = row_loss;
     // lane: N consecutive components, moved as 16-byte vectors (8-byte at dim 64)
 #pragma unroll
     for (int t = 0; t < N; ++t) {
@@ -1061,9 +833,15 @@ __global__ void __launch_bounds__(256) bf16_flush_kernel(const BF16FlushArgs a) 
   }
 }
 
-__global__ void f32_to_bf16_kernel(const float *__restrict__ s, __nv_bfloat16 *__restrict__ d, int64_t n) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    d[i] = __float2bfloat16(s[i]);
+// d = BF16(s), and with m the FP32 rows as well; four values a thread step.
+__global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float4 *__restrict__ s, float4 *__restrict__ m,
+                                                          uint2 *__restrict__ d, int64_t quads) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < quads; i += int64_t(gridDim.x) * blockDim.x) {
+    const float4 v = s[i];
+    if (m) m[i] = v;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    d[i] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+  }
 }
 
 }  // namespace
@@ -1080,10 +858,7 @@ int bf16_repulse_smem_bytes(int dim) {
 namespace {
 template <int D>
 cudaError_t prepare_d() {
-  cudaError_t e = cudaFuncSetAttribute(bf16_repulse_kernel<D, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       RepulseSmem<D>::dynamic);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(bf16_repulse_kernel<D, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(bf16_repulse_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               RepulseSmem<D>::dynamic);
 }
 }  // namespace
@@ -1099,31 +874,7 @@ cudaError_t bf16_prepare(int dim) {
 
 namespace {
 
-// The repulsion GEMMs of a minibatch: one CTA per 128-row tile, or, with at
-// least two chunks of negatives, a cluster of two CTAs per tile that split them.
 template <int D>
-cudaError_t launch_repulse(const BF16BatchArgs &a, const CUtensorMap &mx, const CUtensorMap &mn, int tiles,
-                           cudaStream_t s) {
-  if (a.kpad / kChunk < 2) {
-    bf16_repulse_kernel<D, 1><<<tiles, kRepulseThreads, RepulseSmem<D>::dynamic, s>>>(mx, mn, a);
-    return cudaGetLastError();
-  }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(2 * tiles);
-  cfg.blockDim = dim3(kRepulseThreads);
-  cfg.dynamicSmemBytes = RepulseSmem<D>::dynamic;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, bf16_repulse_kernel<D, 2>, mx, mn, a);
-}
-
-template <int D, int U>
 cudaError_t launch_bf16_batch_d(const BF16BatchArgs &a, const CUtensorMap &mx, const CUtensorMap &mn,
                                 cudaStream_t s, cudaEvent_t *ev, cudaStream_t s2,
                                 cudaEvent_t fork, cudaEvent_t join) {
@@ -1131,14 +882,15 @@ cudaError_t launch_bf16_batch_d(const BF16BatchArgs &a, const CUtensorMap &mx, c
   const int gather_ctas = a.kpad / kGatherTile;  // kpad: a multiple of 64
   const int tiles = (a.rows + kTileRows - 1) / kTileRows;
   const int apply_ctas = (a.rows + 7) / 8;
+  void (*const attract)(BF16BatchArgs) = a.compute_loss ? bf16_attract_kernel<D, true> : bf16_attract_kernel<D, false>;
   cudaError_t e = cudaSuccess;
   if (ev || !s2) {  // one after another (per-kernel timing)
     if (ev) cudaEventRecord(ev[0], s);
     bf16_gather_kernel<D><<<gather_ctas, kGatherTile * 32, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[1], s);
-    bf16_attract_kernel<D, U><<<item_ctas, kPlainWarps * 32, 0, s>>>(a);
+    attract<<<item_ctas, kPlainWarps * 32, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[2], s);
-    if ((e = launch_repulse<D>(a, mx, mn, tiles, s)) != cudaSuccess) return e;
+    bf16_repulse_kernel<D><<<tiles * a.ksplit, kRepulseThreads, RepulseSmem<D>::dynamic, s>>>(mx, mn, a);
     if (ev) cudaEventRecord(ev[3], s);
     bf16_apply_kernel<D><<<apply_ctas, 256, 0, s>>>(a);
     return cudaGetLastError();
@@ -1148,8 +900,8 @@ cudaError_t launch_bf16_batch_d(const BF16BatchArgs &a, const CUtensorMap &mx, c
   // previous minibatch's update and joined before this one's
   if ((e = cudaEventRecord(fork, s)) != cudaSuccess || (e = cudaStreamWaitEvent(s2, fork, 0)) != cudaSuccess) return e;
   bf16_gather_kernel<D><<<gather_ctas, kGatherTile * 32, 0, s2>>>(a);
-  if ((e = launch_repulse<D>(a, mx, mn, tiles, s2)) != cudaSuccess) return e;
-  bf16_attract_kernel<D, U><<<item_ctas, kPlainWarps * 32, 0, s>>>(a);
+  bf16_repulse_kernel<D><<<tiles * a.ksplit, kRepulseThreads, RepulseSmem<D>::dynamic, s2>>>(mx, mn, a);
+  attract<<<item_ctas, kPlainWarps * 32, 0, s>>>(a);
   if ((e = cudaEventRecord(join, s2)) != cudaSuccess || (e = cudaStreamWaitEvent(s, join, 0)) != cudaSuccess) return e;
   bf16_apply_kernel<D><<<apply_ctas, 256, 0, s>>>(a);
   return cudaGetLastError();
@@ -1161,9 +913,9 @@ cudaError_t launch_bf16_batch(int dim, const BF16BatchArgs &a, const CUtensorMap
                               cudaStream_t s, cudaEvent_t *ev, cudaStream_t s2,
                               cudaEvent_t fork, cudaEvent_t join) {
   switch (dim) {
-    case 64: return launch_bf16_batch_d<64, 8>(a, mx, mn, s, ev, s2, fork, join);
-    case 128: return launch_bf16_batch_d<128, 8>(a, mx, mn, s, ev, s2, fork, join);
-    case 256: return launch_bf16_batch_d<256, 4>(a, mx, mn, s, ev, s2, fork, join);
+    case 64: return launch_bf16_batch_d<64>(a, mx, mn, s, ev, s2, fork, join);
+    case 128: return launch_bf16_batch_d<128>(a, mx, mn, s, ev, s2, fork, join);
+    case 256: return launch_bf16_batch_d<256>(a, mx, mn, s, ev, s2, fork, join);
   }
   return cudaErrorInvalidValue;
 }
@@ -1173,10 +925,13 @@ cudaError_t launch_bf16_flush(const BF16FlushArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_f32_to_bf16(const float *src, __nv_bfloat16 *dst, int64_t count, cudaStream_t s) {
+cudaError_t launch_f32_to_bf16(const float *src, __nv_bfloat16 *dst, int64_t count, cudaStream_t s, float *copy) {
   if (count <= 0) return cudaSuccess;
-  const int grid = int(count / 256 + 1 < 152 * 8 ? count / 256 + 1 : 152 * 8);
-  f32_to_bf16_kernel<<<grid, 256, 0, s>>>(src, dst, count);
+  if ((count & 3) || (reinterpret_cast<uintptr_t>(src) & 15)) return cudaErrorInvalidValue;  // whole rows
+  const int64_t quads = count / 4;
+  const int grid = int(quads / 256 + 1 < 152 * 8 ? quads / 256 + 1 : 152 * 8);
+  f32_to_bf16_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const float4 *>(src), reinterpret_cast<float4 *>(copy),
+                                          reinterpret_cast<uint2 *>(dst), quads);
   return cudaGetLastError();
 }
 

@@ -160,7 +160,9 @@ struct BF16BatchArgs {
   float *P;                 // partial slots of split rows
   int32_t *counters;
   float *abuf;              // [B, dim] attractive update of the minibatch (lr applied)
-  float *rbuf;              // [B, dim] repulsive (GEMM) update of the minibatch (lr applied)
+  float *rbuf;              // [ksplit, B, dim] repulsive (GEMM) update of the minibatch (lr applied), in parts
+  double *rloss;            // [ksplit, B] its loss, likewise
+  int32_t ksplit, rstride;  // CTAs that share a tile's negatives; rows of a part (B)
   __nv_bfloat16 *nb;        // [kpad, dim] gathered negatives
   float *nn;                // [kpad] squared norms of the gathered negatives
   int32_t *nid;             // [kpad] vertex id of each negative, -1 = none
@@ -183,6 +185,17 @@ struct BF16FlushArgs {
   int32_t compute_loss;
 };
 
+// CTAs of the repulsion GEMMs to a 128-row tile, for a minibatch of `rows` rows and kpad
+// gathered negatives: as many as still run at once (one CTA an SM), with at least two
+// 64-negative chunks each, four at most.  Measured, us a launch at one / two / four CTAs
+// a tile: 64 tiles, 16 chunks, dim 256 30.8 / 22.5; 16 tiles, 16 chunks, dim 128 24.7 /
+// 16.5 / 13.1; 8 tiles, 8 chunks, dim 256 20.5 / 16.4 / 14.3; 32 tiles, 4 chunks, dim 128
+// 13.3 / 12.2.
+inline int bf16_ksplit(int64_t rows, int64_t kpad) {
+  const int64_t tiles = (rows + 127) / 128, chunks = kpad / 64;
+  return int(std::max<int64_t>(1, std::min<int64_t>({152 / tiles, chunks / 2, int64_t(4)})));
+}
+
 // BF16 launchers (de_bf16.cu).
 int bf16_repulse_smem_bytes(int dim);
 cudaError_t bf16_prepare(int dim);
@@ -195,7 +208,9 @@ cudaError_t launch_bf16_batch(int dim, const BF16BatchArgs &a, const CUtensorMap
                               cudaStream_t s, cudaEvent_t *ev, cudaStream_t s2,
                               cudaEvent_t fork, cudaEvent_t join);
 cudaError_t launch_bf16_flush(const BF16FlushArgs &a, cudaStream_t s);
-cudaError_t launch_f32_to_bf16(const float *src, __nv_bfloat16 *dst, int64_t count, cudaStream_t s);
+// dst = BF16(src) and, with copy, copy = src; whole rows, src on a 16-byte boundary
+cudaError_t launch_f32_to_bf16(const float *src, __nv_bfloat16 *dst, int64_t count, cudaStream_t s,
+                               float *copy = nullptr);
 
 // Where a handle's buffers come from.  With dalloc set, device buffers come from
 // dalloc/dfree (a caller-owned arena; no implicit device synchronisation) and

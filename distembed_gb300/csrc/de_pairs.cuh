@@ -1,5 +1,5 @@
 // The pairs of a work item with its rows' addresses held by the warp's lanes, shared by
-// the FP32 plain, SpMM and sparse embedding kernels.
+// the FP32 plain, SpMM, sparse embedding and BF16 attractive kernels.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -20,14 +20,17 @@ struct Lay {
   static constexpr int LP = D >= 128 ? 32 : D / 8, G = 32 / LP, C = D / LP;
   static constexpr int S = D == 128 ? 8 : D == 256 ? 4 : 2;
 };
-template <int D>
-struct LaneRow {
-  float v[Lay<D>::C];
+// A lane's components of a row.
+template <int N>
+struct LaneVec {
+  float v[N];
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int t = 0; t < Lay<D>::C; ++t) v[t] = 0.f;
+    for (int t = 0; t < N; ++t) v[t] = 0.f;
   }
 };
+template <int D>
+using LaneRow = LaneVec<Lay<D>::C>;
 
 // How a row is read: kFinal, rows that no launch in flight writes (read-only path);
 // kStaged, rows of minibatch j-1 written by the launch before (L2); kShared, shared
@@ -56,14 +59,49 @@ __device__ __forceinline__ void store_lanes(const LaneRow<D> &f, float *row, int
   }
 }
 
-// The lane groups' sums of a row added up (fixed order), on every lane.
+// The sums of a row's lane groups of LP added up (fixed order), on every lane.
+template <int LP, int C>
+__device__ __forceinline__ void sum_lane_groups(LaneVec<C> &acc) {
+#pragma unroll
+  for (int m = LP; m < 32; m <<= 1)
+#pragma unroll
+    for (int t = 0; t < C; ++t) acc.v[t] += __shfl_xor_sync(kFull, acc.v[t], m);
+}
 template <int D>
 __device__ __forceinline__ void sum_groups(LaneRow<D> &acc) {
-#pragma unroll
-  for (int m = Lay<D>::LP; m < 32; m <<= 1)
-#pragma unroll
-    for (int t = 0; t < Lay<D>::C; ++t) acc.v[t] += __shfl_xor_sync(kFull, acc.v[t], m);
+  sum_lane_groups<Lay<D>::LP>(acc);
 }
+
+// What the pair loops need to know of the rows: the layout above, how a lane's share of
+// a row is loaded and kept until it is used (Raw), and how it becomes FP32.
+template <int D, RowRead kRead>
+struct F32Rows {
+  static constexpr int LP = Lay<D>::LP, G = Lay<D>::G, C = Lay<D>::C, S = Lay<D>::S;
+  typedef LaneRow<D> Raw;
+  static __device__ __forceinline__ void load(Raw &x, const void *row, int gl) {
+    load_lanes<D, kRead>(x, static_cast<const float *>(row), gl);
+  }
+  static __device__ __forceinline__ const LaneVec<C> &unpack(const Raw &x) { return x; }
+};
+// BF16 rows: 16 bytes (8 components in order) a lane.
+template <int D, int kSteps>
+struct B16Rows {
+  static constexpr int LP = D / 8, G = 32 / LP, C = 8, S = kSteps;
+  typedef uint4 Raw;
+  static __device__ __forceinline__ void load(Raw &x, const void *row, int gl) {
+    x = __ldg(static_cast<const uint4 *>(row) + gl);
+  }
+  static __device__ __forceinline__ LaneVec<C> unpack(const Raw &x) {
+    LaneVec<C> f;
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      f.v[2 * i] = __uint_as_float(w[i] << 16);
+      f.v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+    return f;
+  }
+};
 
 // What an item's pairs share.
 struct PairCtx {
@@ -82,21 +120,21 @@ struct PairCtx {
 // other row.  Bit k of vm: pair k counts, of rm: it counts and repels.  The row of a
 // pair that does not count is x_i's own, whose (attractive) force is exactly 0.
 // Attractive: c = -2/(1+r); repulsive: c = 2/((r+1e-6)(1+r)) (algo.hpp:573, 626/641).
-template <int D, int S, RowRead kRead>
-__device__ __forceinline__ void pair_steps(LaneRow<D> &acc, const LaneRow<D> &xi, const float *rows, unsigned vm,
+template <class R, int S>
+__device__ __forceinline__ void pair_steps(LaneVec<R::C> &acc, const LaneVec<R::C> &xi, const void *rows, unsigned vm,
                                            unsigned rm, int k0, const PairCtx &c, float &loss, int lane) {
-  constexpr int LP = Lay<D>::LP, G = Lay<D>::G, C = Lay<D>::C;
+  constexpr int LP = R::LP, G = R::G, C = R::C;
   const int q = G > 1 ? lane / LP : 0, gl = G > 1 ? lane % LP : lane;
-  LaneRow<D> x[S];
+  typename R::Raw raw[S];
 #pragma unroll
-  for (int s = 0; s < S; ++s) {
-    const float *row = reinterpret_cast<const float *>(
-        __shfl_sync(kFull, reinterpret_cast<unsigned long long>(rows), k0 + s * G + q));
-    load_lanes<D, kRead>(x[s], row, gl);
-  }
+  for (int s = 0; s < S; ++s)
+    R::load(raw[s], reinterpret_cast<const void *>(
+                        __shfl_sync(kFull, reinterpret_cast<unsigned long long>(rows), k0 + s * G + q)), gl);
+  LaneVec<C> x[S];  // x_i - the row
   float r[S];
 #pragma unroll
   for (int s = 0; s < S; ++s) {
+    x[s] = R::unpack(raw[s]);
     float2 p = make_float2(0.f, 0.f);
 #pragma unroll
     for (int t = 0; t < C; t += 2) {
@@ -155,15 +193,15 @@ __device__ __forceinline__ void pair_steps(LaneRow<D> &acc, const LaneRow<D> &xi
 }
 
 // Every pair of a window of 32, S steps at a time and half as many at its end.
-template <int D, RowRead kRead, int S = Lay<D>::S>
-__device__ __forceinline__ void pair_window(LaneRow<D> &acc, const LaneRow<D> &xi, const float *rows, unsigned vm,
+template <class R, int S = R::S>
+__device__ __forceinline__ void pair_window(LaneVec<R::C> &acc, const LaneVec<R::C> &xi, const void *rows, unsigned vm,
                                             unsigned rm, const PairCtx &c, float &loss, int lane) {
-  constexpr int kChunk = S * Lay<D>::G;
+  constexpr int kChunk = S * R::G;
   const int end = 32 - __clz(vm);
   for (int k = 0; k < end; k += kChunk) {
     if (((vm >> k) & (kFull >> (32 - kChunk))) == 0) continue;
-    if (end - k > kChunk / 2) pair_steps<D, S, kRead>(acc, xi, rows, vm, rm, k, c, loss, lane);
-    else pair_steps<D, S / 2, kRead>(acc, xi, rows, vm, rm, k, c, loss, lane);
+    if (end - k > kChunk / 2) pair_steps<R, S>(acc, xi, rows, vm, rm, k, c, loss, lane);
+    else pair_steps<R, S / 2>(acc, xi, rows, vm, rm, k, c, loss, lane);
   }
 }
 

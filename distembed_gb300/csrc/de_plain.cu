@@ -166,9 +166,9 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kMinBlocks<D>)
     const float *row = now ? row_ptr<false>(a, ids, D) : own;
     if (a.stage_negs) {
       if (repels) row = negsm + (k0 + lane - cnt) * D;
-      pair_window<D, kShared>(acc, xi, row, vm, rm, c, loss, lane);
+      pair_window<F32Rows<D, kShared>>(acc, xi, row, vm, rm, c, loss, lane);
     } else {
-      pair_window<D, kFinal>(acc, xi, row, vm, rm, c, loss, lane);
+      pair_window<F32Rows<D, kFinal>>(acc, xi, row, vm, rm, c, loss, lane);
     }
   }
   pdl_wait();
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kMinBlocks<D>)
     if (total > 32) ids = fetch(k0);
     const bool late = ids >= 0 && in_prev(a, ids);
     const unsigned vm = __ballot_sync(kFull, late), rm = __ballot_sync(kFull, late && k0 + lane >= cnt);
-    if (vm) pair_window<D, kStaged>(acc, xi, late ? row_ptr<true>(a, ids, D) : own, vm, rm, c, loss, lane);
+    if (vm) pair_window<F32Rows<D, kStaged>>(acc, xi, late ? row_ptr<true>(a, ids, D) : own, vm, rm, c, loss, lane);
   }
   if (has_item) {
     sum_groups<D>(acc);
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kTeamMinBlocks<D>)
     const float *row = now ? row_ptr<false>(a, ids, D) : own;
     for (int r = 0; r < kGroups && s + r < mine; ++r)
       if ((vm >> (r * kPairs)) & ((1u << kPairs) - 1))
-        pair_steps<D, kSteps, kFinal>(acc, xi, row, vm, rm, r * kPairs, c, loss, lane);
+        pair_steps<F32Rows<D, kFinal>, kSteps>(acc, xi, row, vm, rm, r * kPairs, c, loss, lane);
   }
   pdl_wait();
   pdl_trigger();
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kTeamMinBlocks<D>)
     const float *row = late ? row_ptr<true>(a, ids, D) : own;
     for (int r = 0; vm != 0 && r < kGroups && s + r < mine; ++r)
       if ((vm >> (r * kPairs)) & ((1u << kPairs) - 1))
-        pair_steps<D, kSteps, kStaged>(acc, xi, row, vm, rm, r * kPairs, c, loss, lane);
+        pair_steps<F32Rows<D, kStaged>, kSteps>(acc, xi, row, vm, rm, r * kPairs, c, loss, lane);
   }
   sum_groups<D>(acc);
   if (c.want_loss) {

@@ -136,7 +136,9 @@ int64_t job_bytes(const de_job_spec &s) {
   b += 8 * 2048;                                                        // small fixed buffers
   if (s.precision == DE_PRECISION_BF16) {
     const int64_t kpad = std::max<int64_t>(64, (s.ns + 63) / 64 * 64);
-    b += 2 * n * D + 8 * n + 2 * B * D * 4 + 2 * kpad * D * 2 + kpad * 8 + B * 32 * 4;  // + update rows
+    const int64_t parts = de::bf16_ksplit(std::min(n, B), kpad);
+    b += 2 * n * D + 8 * n + (1 + parts) * B * D * 4 + parts * B * 8;  // + update rows and their losses
+    b += 2 * kpad * D * 2 + kpad * 8 + B * 32 * 4;
   }
   return b + b / 16 + (1 << 20);  // allocator rounding and slack
 }

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kAttractMinBlocks<D>) sparse
     dev::LaneRow<D> xi, sum;
     dev::load_lanes<D, dev::kFinal>(xi, own, lane);
     sum.zero();
-    dev::pair_window<D, dev::kFinal, 4>(sum, xi, id >= 0 ? a.X + size_t(id) * D : own, __ballot_sync(kFull, id >= 0), 0u,
+    dev::pair_window<dev::F32Rows<D, dev::kFinal>, 4>(sum, xi, id >= 0 ? a.X + size_t(id) * D : own, __ballot_sync(kFull, id >= 0), 0u,
                                      c, unused_loss, lane);
 #pragma unroll
     for (int t = 0; t < Frag<D>::N; ++t) acc.v[t] = sum.v[t];
