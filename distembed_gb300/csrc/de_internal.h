@@ -107,6 +107,7 @@ struct PlainBatchArgs {
   int32_t *err;             // set when a bounded device wait gives up
 };
 
+constexpr int kStageSlots = 4;   // staging buffers of the FP32 plain form, a ring over the minibatches
 constexpr int kStageNegMax = 8;  // negatives per minibatch the shared-memory staging takes
 
 struct FlushArgs {

@@ -51,7 +51,7 @@ struct de_handle {
 
   // per-minibatch-size state
   Schedule sched;
-  float *d_stage = nullptr;  // three minibatch staging buffers
+  float *d_stage = nullptr;  // kStageSlots minibatch staging buffers
   float *d_y = nullptr;      // SpMM output [n, dim]
   int32_t *d_spmm_off = nullptr;  // SpMM: per-minibatch first partial slot, then first counter
   int spmm_batch = 0, spmm_cap = 0;
@@ -458,9 +458,9 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
     PlainBatchArgs a{};
     a.X = h->d_x;
     const size_t slice = size_t(s.batch) * h->dim;
-    a.S_cur = h->d_stage + slice * (j % 3);
-    a.S_prev = h->d_stage + slice * ((j + 2) % 3);
-    a.S_prev2 = h->d_stage + slice * ((j + 1) % 3);
+    a.S_cur = h->d_stage + slice * (j % kStageSlots);
+    a.S_prev = h->d_stage + slice * ((j + kStageSlots - 1) % kStageSlots);
+    a.S_prev2 = h->d_stage + slice * ((j + kStageSlots - 2) % kStageSlots);
     a.rowptr = h->d_rowptr;
     a.col = h->d_col;
     a.items = s.d_items + s.item_off[j];
@@ -497,7 +497,7 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
   if (err == cudaSuccess) {
     FlushArgs f{};
     f.X = h->d_x;
-    f.S_last = h->d_stage + size_t(s.batch) * h->dim * ((s.batches - 1) % 3);
+    f.S_last = h->d_stage + size_t(s.batch) * h->dim * ((s.batches - 1) % kStageSlots);
     f.last_base = int32_t(int64_t(s.batches - 1) * s.batch);
     f.last_rows = s.last_batch_size;
     f.loss_partial = h->d_loss_partial;
@@ -887,7 +887,7 @@ static int prepare_run(de_handle *h, int32_t first_epoch, int32_t epochs, int32_
   bool moved = false;
   int rc = DE_OK;
   const bool bf16 = h->opt.precision == DE_PRECISION_BF16;
-  if (!bf16 && (rc = grow(h, &h->d_stage, &h->stage_cap, size_t(3) * s.batch * h->dim, &moved)) != DE_OK) return rc;
+  if (!bf16 && (rc = grow(h, &h->d_stage, &h->stage_cap, size_t(kStageSlots) * s.batch * h->dim, &moved)) != DE_OK) return rc;
   if (bf16 && (rc = ensure_bf16_buffers(h, ns, &moved)) != DE_OK) return rc;
   bool counters_moved = false;
   if ((rc = grow(h, &h->d_parts, &h->parts_cap, size_t(std::max(s.max_parts, 1)) * h->dim, &moved)) ||

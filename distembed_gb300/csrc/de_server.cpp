@@ -130,7 +130,7 @@ int64_t job_bytes(const de_job_spec &s) {
   }
   int64_t b = 4 * (n + 1) + 4 * std::max<int64_t>(nnz, 1) + 4 * n * D;  // CSR, embedding
   b += 32 * items;                                                      // work items
-  b += 3 * B * D * 4 + max_items * D * 4 + max_items * 4;               // staging, partial slots, counters
+  b += de::kStageSlots * B * D * 4 + max_items * D * 4 + max_items * 4;               // staging, partial slots, counters
   b += 8 * items;                                                       // per-item loss partials
   b += int64_t(s.epochs) * (batches * s.ns * 4 + 16);                   // negatives, rates, losses
   b += 8 * 2048;                                                        // small fixed buffers
