@@ -102,6 +102,8 @@ struct PlainBatchArgs {
   double *loss_partial;     // one per work item of the epoch
   int64_t loss_off;         // first item of this minibatch in the epoch
   const int32_t *epoch;     // device [2]: epoch index within this call, first epoch of the call
+  int32_t epoch_at, first_epoch_at;  // epoch_at >= 0: these and lr_at are used instead of epoch and lr
+  float lr_at;
   int32_t stage_negs;       // 1: the minibatch's final negative rows are copied into every CTA's
                             // shared memory (cp.async.bulk) before the repulsive pass; ns <= kStageNegMax
   int32_t *err;             // set when a bounded device wait gives up
@@ -125,6 +127,18 @@ struct FlushArgs {
 
 constexpr int kFlushBlocks = 152;
 constexpr int64_t kFlushChunk = 2048;  // loss partials of a CTA at least: eight a thread, one round of loads
+// Loss partials a CTA sums, and the CTAs that makes.
+__host__ __device__ inline int64_t flush_chunk(int64_t n_partials) {
+  const int64_t per = (n_partials + kFlushBlocks - 1) / kFlushBlocks;
+  return per > kFlushChunk ? per : kFlushChunk;
+}
+__host__ __device__ inline int flush_parts(int64_t n_partials) {
+  const int64_t chunk = flush_chunk(n_partials);
+  return int((n_partials + chunk - 1) / chunk);
+}
+// Epochs of one minibatch: per-item losses kept at once for several epochs (an epoch of
+// more items stands alone).
+constexpr int64_t kEpochLossItems = int64_t(1) << 18;
 
 // The SpMM step (spmm_kernel): every work item of every minibatch in one launch,
 // y rows from the unchanged input x; a minibatch's split rows use partial slots
@@ -239,6 +253,10 @@ cudaError_t launch_columns(const int64_t *src, int32_t *dst, int64_t count, int6
 // teams: several warps to a work item where plain_team_warps says so (one otherwise).
 cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, bool teams, bool pdl, cudaStream_t s);
 cudaError_t launch_flush(int dim, const FlushArgs &a, bool pdl, cudaStream_t s);
+// loss[e] for e in [0, epochs) from partial [epochs, n_items], summed as launch_flush does;
+// block_sums: epochs * flush_parts(n_items) values.
+cudaError_t launch_epoch_losses(const double *partial, int64_t n_items, int epochs, double *block_sums, double *loss,
+                                cudaStream_t s);
 cudaError_t launch_spmm(int dim, const SpmmArgs &a, cudaStream_t s);
 
 // Sparse embedding (de_sparse.cu).  Rows are FP64 vectors with INT_MIN marking

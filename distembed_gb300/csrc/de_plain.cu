@@ -37,6 +37,14 @@ namespace {
 
 using namespace dev;
 
+__device__ __forceinline__ int epoch_of(const PlainBatchArgs &a) { return a.epoch_at >= 0 ? a.epoch_at : a.epoch[0]; }
+__device__ __forceinline__ int first_epoch_of(const PlainBatchArgs &a) {
+  return a.epoch_at >= 0 ? a.first_epoch_at : a.epoch[1];
+}
+__device__ __forceinline__ float rate_of(const PlainBatchArgs &a, int epoch) {
+  return a.epoch_at >= 0 ? a.lr_at : a.lr[epoch];
+}
+
 __device__ __forceinline__ bool in_prev(const PlainBatchArgs &a, int n) {
   return unsigned(n - a.prev_base) < unsigned(a.prev_rows);
 }
@@ -122,12 +130,12 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kMinBlocks<D>)
   const bool has_item = gw < a.n_items;
   WorkItem it{};
   if (has_item) it = a.items[gw];
-  const int epoch = a.epoch[0];
-  const PairCtx c(a.lr[epoch], a.bound, a.compute_loss != 0);
+  const int epoch = epoch_of(a);
+  const PairCtx c(rate_of(a, epoch), a.bound, a.compute_loss != 0);
   const int skip = a.skip_last ? a.n - 1 : -1;  // edges into n-1 are dropped (algo.hpp:399-405, 538)
   const int cnt = it.e_end - it.e_begin;
   // the repulsive pass of a row is done by its part 0
-  const int rep_rows = (a.quirks && epoch + a.epoch[1] > 0) ? a.last_batch_size : a.rows;
+  const int rep_rows = (a.quirks && epoch + first_epoch_of(a) > 0) ? a.last_batch_size : a.rows;
   const int total = cnt + (has_item && it.part == 0 && it.row < rep_rows ? a.ns : 0);
   const int32_t *negs = a.negs + (size_t(epoch) * a.batches + a.batch_id) * a.ns;
   // the other row of the item's pair k0 + lane: its CSR entries, then the draws; -1 = none
@@ -238,16 +246,19 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kTeamMinBlocks<D>)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int team = warp / W, tw = warp % W;
   const int item = blockIdx.x * kTeams + team;
-  if (a.first) pdl_wait();  // as in plain_batch_kernel
+  if (a.first) {  // as in plain_batch_kernel
+    pdl_wait();
+    pdl_trigger();
+  }
   const bool has_item = item < a.n_items;
   WorkItem it{};
   if (has_item) it = a.items[item];
-  const int epoch = a.epoch[0];
-  const PairCtx c(a.lr[epoch], a.bound, a.compute_loss != 0);
+  const int epoch = epoch_of(a);
+  const PairCtx c(rate_of(a, epoch), a.bound, a.compute_loss != 0);
   const int skip = a.skip_last ? a.n - 1 : -1;  // edges into n-1 are dropped (algo.hpp:399-405, 538)
   const int cnt = it.e_end - it.e_begin;
   // the repulsive pass of a row is done by its part 0
-  const int rep_rows = (a.quirks && epoch + a.epoch[1] > 0) ? a.last_batch_size : a.rows;
+  const int rep_rows = (a.quirks && epoch + first_epoch_of(a) > 0) ? a.last_batch_size : a.rows;
   const int total = cnt + (has_item && it.part == 0 && it.row < rep_rows ? a.ns : 0);
   const int32_t *negs = a.negs + (size_t(epoch) * a.batches + a.batch_id) * a.ns;
   const int groups = (total + kPairs - 1) / kPairs;
@@ -442,9 +453,8 @@ __global__ void __launch_bounds__(256) flush_kernel(const FlushArgs a) {
   }
   // The loss: kFlushChunk partials a CTA (or more, where the grid is too small), so
   // a small job's sum needs no second step across CTAs.
-  const int64_t per = (a.n_partials + gridDim.x - 1) / gridDim.x;
-  const int64_t chunk = per > kFlushChunk ? per : kFlushChunk;
-  const int parts = int((a.n_partials + chunk - 1) / chunk);
+  const int64_t chunk = flush_chunk(a.n_partials);
+  const int parts = flush_parts(a.n_partials);
   if (int(blockIdx.x) >= parts) return;
   __shared__ double red[8];
   __shared__ bool last;
@@ -467,6 +477,21 @@ __global__ void __launch_bounds__(256) flush_kernel(const FlushArgs a) {
     a.epoch[0] = e + 1;
     *a.done = 0;
   }
+}
+
+// Losses of epochs (blockIdx.x) whose items' losses lie one epoch after another: with
+// one part (blockIdx.y) the sum, else the parts' sums for epoch_parts_kernel; in
+// flush_kernel's order.
+__global__ void __launch_bounds__(256) epoch_losses_kernel(const double *partial, int64_t n_items, double *out) {
+  __shared__ double red[8];
+  const int64_t chunk = flush_chunk(n_items), lo = blockIdx.y * chunk;
+  const double s = block_sum(partial + int64_t(blockIdx.x) * n_items + lo, min(n_items - lo, chunk), red);
+  if (threadIdx.x == 0) out[int64_t(blockIdx.x) * gridDim.y + blockIdx.y] = s;
+}
+__global__ void __launch_bounds__(256) epoch_parts_kernel(const double *sums, int parts, double *loss) {
+  __shared__ double red[8];
+  const double s = block_sum(sums + int64_t(blockIdx.x) * parts, parts, red);
+  if (threadIdx.x == 0) loss[blockIdx.x] = s;
 }
 
 __global__ void f64_to_f32_kernel(const double *__restrict__ s, float *__restrict__ d, int64_t n) {
@@ -530,6 +555,14 @@ cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, bool teams, boo
     case 256: return launch(plain_batch_kernel<256>, grid, block, a, pdl, s, smem);
     default: return cudaErrorInvalidValue;
   }
+}
+
+cudaError_t launch_epoch_losses(const double *partial, int64_t n_items, int epochs, double *block_sums, double *loss,
+                                cudaStream_t s) {
+  const int parts = flush_parts(n_items);
+  epoch_losses_kernel<<<dim3(epochs, parts), 256, 0, s>>>(partial, n_items, parts > 1 ? block_sums : loss);
+  if (parts > 1) epoch_parts_kernel<<<epochs, 256, 0, s>>>(block_sums, parts, loss);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_spmm(int dim, const SpmmArgs &a, cudaStream_t s) {

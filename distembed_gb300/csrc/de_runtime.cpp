@@ -72,7 +72,8 @@ struct de_handle {
   size_t counters_cap = 0;
   double *d_loss_partial = nullptr;
   size_t loss_partial_cap = 0;
-  double *d_block_sums = nullptr;  // [kFlushBlocks]
+  double *d_block_sums = nullptr;  // [kFlushBlocks], more for several epochs at once
+  size_t block_sums_cap = 0;
   int32_t *d_done = nullptr;       // flush arrival counter
 
   // per-call state
@@ -448,6 +449,79 @@ int ensure_bf16_buffers(de_handle *h, int ns, bool *moved) {
   return DE_OK;
 }
 
+// The arguments every minibatch of the FP32 plain form shares.
+PlainBatchArgs plain_args(const de_handle *h, int ns) {
+  const Schedule &s = h->sched;
+  PlainBatchArgs a{};
+  a.X = h->d_x;
+  a.rowptr = h->d_rowptr;
+  a.col = h->d_col;
+  a.batches = s.batches;
+  a.last_batch_size = s.last_batch_size;
+  a.n = int32_t(h->n);
+  a.quirks = h->opt.ref_quirks;
+  a.skip_last = h->opt.ref_quirks && !h->keep_last_edges;
+  a.compute_loss = h->opt.compute_loss;
+  a.bound = float(h->opt.max_bound);
+  a.negs = h->d_negs;
+  a.ns = ns;
+  a.lr = h->d_lr;
+  a.P = h->d_parts;
+  a.counters = h->d_counters;
+  a.loss_partial = h->d_loss_partial;
+  a.epoch = h->d_epoch;
+  a.epoch_at = -1;
+  a.stage_negs = h->opt.stage_negatives && ns > 0 && ns <= kStageNegMax;
+  a.err = h->d_err;
+  return a;
+}
+
+// Several warps to a work item where it is small (plain_team_warps); a caller that sets
+// the edge cap asks for one warp a work item of that size.
+bool item_teams(const de_handle *h, const PlainBatchArgs &a) { return h->opt.edge_cap <= 0 && !a.stage_negs; }
+
+// Rows of a staging buffer, and how many an epoch of the schedule uses.
+size_t stage_rows(const Schedule &s, int64_t n) { return size_t(std::min<int64_t>(s.batch, n)); }
+size_t stage_slots(const Schedule &s) { return size_t(std::min(s.batches, kStageSlots)); }
+
+// Epochs of one minibatch whose per-item losses are kept at once.
+int loss_epochs(const de_handle *h, int epochs) {
+  return int(std::min<int64_t>(epochs, std::max<int64_t>(1, kEpochLossItems / std::max<int64_t>(1, h->sched.n_items))));
+}
+
+// Enqueues the epochs of a run whose minibatch is the whole graph.  Epoch e reads one of
+// two embeddings and writes every row of the other (d_x and the staging buffer), so an
+// epoch is one launch: no copy back, no flush, the epoch's index and rate in its
+// arguments, and the losses of many epochs summed by one launch at the end.  1,507
+// vertices, dim 32, 20 epochs with loss: 285 -> 208 us a run from host rows.
+cudaError_t enqueue_whole_graph(de_handle *h, int first_epoch, int epochs, int ns, const double *lr) {
+  const Schedule &s = h->sched;
+  PlainBatchArgs a = plain_args(h, ns);
+  a.items = s.d_items;
+  a.n_items = int32_t(s.n_items);
+  a.rows = int32_t(h->n);
+  a.first = 1;
+  a.first_epoch_at = first_epoch;
+  float *from = h->d_x, *to = h->d_stage;
+  const int keep = loss_epochs(h, epochs);
+  cudaError_t err = cudaSuccess;
+  for (int e = 0; e < epochs && err == cudaSuccess; ++e) {
+    a.X = from;
+    a.S_cur = to;
+    a.epoch_at = e;
+    a.lr_at = float(lr[e]);
+    a.loss_off = int64_t(e % keep) * s.n_items;
+    err = launch_plain_batch(h->dim, a, item_teams(h, a), h->opt.pdl != 0, h->stream);
+    std::swap(from, to);
+    if (err == cudaSuccess && h->opt.compute_loss && (e % keep == keep - 1 || e == epochs - 1))
+      err = launch_epoch_losses(h->d_loss_partial, s.n_items, e % keep + 1, h->d_block_sums, h->d_loss + (e - e % keep),
+                                h->stream);
+  }
+  if (err == cudaSuccess && from != h->d_x)
+    err = cudaMemcpyAsync(h->d_x, from, size_t(h->n) * h->dim * sizeof(float), cudaMemcpyDeviceToDevice, h->stream);
+  return err;
+}
+
 // Enqueues one epoch of the FP32 plain form on st.  ev (nullable): one event
 // before each minibatch launch and one before the flush (the events also stop
 // launches from overlapping).
@@ -455,14 +529,11 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
   const Schedule &s = h->sched;
   cudaError_t err = cudaSuccess;
   for (int j = 0; j < s.batches && err == cudaSuccess; ++j) {
-    PlainBatchArgs a{};
-    a.X = h->d_x;
-    const size_t slice = size_t(s.batch) * h->dim;
+    PlainBatchArgs a = plain_args(h, ns);
+    const size_t slice = stage_rows(s, h->n) * h->dim;
     a.S_cur = h->d_stage + slice * (j % kStageSlots);
     a.S_prev = h->d_stage + slice * ((j + kStageSlots - 1) % kStageSlots);
     a.S_prev2 = h->d_stage + slice * ((j + kStageSlots - 2) % kStageSlots);
-    a.rowptr = h->d_rowptr;
-    a.col = h->d_col;
     a.items = s.d_items + s.item_off[j];
     a.n_items = int32_t(s.item_off[j + 1] - s.item_off[j]);
     a.base = int32_t(int64_t(j) * s.batch);
@@ -473,31 +544,14 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
     a.prev2_rows = j > 1 ? s.batch : 0;
     a.batch_id = j;
     a.first = j == 0;
-    a.batches = s.batches;
-    a.last_batch_size = s.last_batch_size;
-    a.n = int32_t(h->n);
-    a.quirks = h->opt.ref_quirks;
-    a.skip_last = h->opt.ref_quirks && !h->keep_last_edges;
-    a.compute_loss = h->opt.compute_loss;
-    a.bound = float(h->opt.max_bound);
-    a.negs = h->d_negs;
-    a.ns = ns;
-    a.lr = h->d_lr;
-    a.P = h->d_parts;
-    a.counters = h->d_counters;
-    a.loss_partial = h->d_loss_partial;
     a.loss_off = s.item_off[j];
-    a.epoch = h->d_epoch;
-    a.stage_negs = h->opt.stage_negatives && ns > 0 && ns <= kStageNegMax;
-    a.err = h->d_err;
     if (ev) cudaEventRecord(ev[j], st);
-    // a caller that sets the edge cap asks for one warp a work item of that size
-    err = launch_plain_batch(h->dim, a, h->opt.edge_cap <= 0 && !a.stage_negs, h->opt.pdl && !ev, st);
+    err = launch_plain_batch(h->dim, a, item_teams(h, a), h->opt.pdl && !ev, st);
   }
   if (err == cudaSuccess) {
     FlushArgs f{};
     f.X = h->d_x;
-    f.S_last = h->d_stage + size_t(s.batch) * h->dim * ((s.batches - 1) % kStageSlots);
+    f.S_last = h->d_stage + stage_rows(s, h->n) * h->dim * ((s.batches - 1) % kStageSlots);
     f.last_base = int32_t(int64_t(s.batches - 1) * s.batch);
     f.last_rows = s.last_batch_size;
     f.loss_partial = h->d_loss_partial;
@@ -533,8 +587,8 @@ cudaError_t enqueue_epoch(de_handle *h, int ns, cudaStream_t st, cudaEvent_t *ev
 // Epochs of at most this many minibatches are launched kernel by kernel: a graph
 // launch per epoch costs more than two to five launches that overlap, and its
 // capture falls away from the first run.  Measured, 10 to 20 epochs, dim 32, us a
-// run by graph -> by launches: 1 minibatch 272 -> 210 (first run 466 -> 395),
-// 3 441 -> 437 (1335 -> 1293), 8 642 -> 647, 34 1351 -> 1442.
+// run by graph -> by launches: 3 minibatches 441 -> 437 (first run 1335 -> 1293), 8
+// 642 -> 647, 34 1351 -> 1442.  One minibatch has a form of its own (enqueue_whole_graph).
 constexpr int kDirectBatches = 4;
 
 int capture_epoch(de_handle *h, int ns) {
@@ -651,6 +705,7 @@ int create_handle(int64_t n, const int64_t *rowptr, const int64_t *col, int64_t 
   h->nnz = nnz;
   h->dim = dim;
   h->device = h->opt.device;
+  h->block_sums_cap = kFlushBlocks;
   h->rowptr.assign(rowptr, rowptr + n + 1);
 
   auto bail = [&](int rc) {
@@ -887,12 +942,15 @@ static int prepare_run(de_handle *h, int32_t first_epoch, int32_t epochs, int32_
   bool moved = false;
   int rc = DE_OK;
   const bool bf16 = h->opt.precision == DE_PRECISION_BF16;
-  if (!bf16 && (rc = grow(h, &h->d_stage, &h->stage_cap, size_t(kStageSlots) * s.batch * h->dim, &moved)) != DE_OK) return rc;
+  if (!bf16 && (rc = grow(h, &h->d_stage, &h->stage_cap, stage_slots(s) * stage_rows(s, h->n) * h->dim, &moved)) != DE_OK) return rc;
   if (bf16 && (rc = ensure_bf16_buffers(h, ns, &moved)) != DE_OK) return rc;
   bool counters_moved = false;
+  const int keep = !bf16 && s.batches == 1 && h->opt.compute_loss ? loss_epochs(h, epochs) : 1;
   if ((rc = grow(h, &h->d_parts, &h->parts_cap, size_t(std::max(s.max_parts, 1)) * h->dim, &moved)) ||
       (rc = grow(h, &h->d_counters, &h->counters_cap, size_t(std::max(s.max_split, 1)), &counters_moved)) ||
-      (rc = grow(h, &h->d_loss_partial, &h->loss_partial_cap, size_t(s.n_items), &moved)))
+      (rc = grow(h, &h->d_loss_partial, &h->loss_partial_cap, size_t(keep) * s.n_items, &moved)) ||
+      (rc = grow(h, &h->d_block_sums, &h->block_sums_cap,
+                 std::max<size_t>(kFlushBlocks, size_t(keep) * flush_parts(s.n_items)), &moved)))
     return rc;
   if (counters_moved) {
     DE_CUDA(h, cudaMemsetAsync(h->d_counters, 0, h->counters_cap * sizeof(int32_t), h->stream));
@@ -945,7 +1003,9 @@ int de_run_from(de_handle *h, int32_t first_epoch, int32_t epochs, int32_t batch
   int rc = prepare_run(h, first_epoch, epochs, batch_size, ns, lr_per_epoch);
   if (rc) return rc;
   const Schedule &s = h->sched;
-  if (h->opt.precision == DE_PRECISION_FP32 && s.batches <= kDirectBatches) {
+  if (h->opt.precision == DE_PRECISION_FP32 && s.batches == 1) {
+    DE_CUDA(h, enqueue_whole_graph(h, first_epoch, epochs, ns, lr_per_epoch));
+  } else if (h->opt.precision == DE_PRECISION_FP32 && s.batches <= kDirectBatches) {
     for (int i = 0; i < epochs; ++i) DE_CUDA(h, enqueue_epoch(h, ns, h->stream, nullptr));
   } else {
     if (!h->graph || h->graph_batch != s.batch || h->graph_ns != ns) {

@@ -131,7 +131,8 @@ int64_t job_bytes(const de_job_spec &s) {
   int64_t b = 4 * (n + 1) + 4 * std::max<int64_t>(nnz, 1) + 4 * n * D;  // CSR, embedding
   b += 32 * items;                                                      // work items
   b += de::kStageSlots * B * D * 4 + max_items * D * 4 + max_items * 4;               // staging, partial slots, counters
-  b += 8 * items;                                                       // per-item loss partials
+  // per-item loss partials, of several epochs when the minibatch is the whole graph
+  b += 8 * (batches > 1 ? items : std::max(items, std::min(items * s.epochs, de::kEpochLossItems)));
   b += int64_t(s.epochs) * (batches * s.ns * 4 + 16);                   // negatives, rates, losses
   b += 8 * 2048;                                                        // small fixed buffers
   if (s.precision == DE_PRECISION_BF16) {
