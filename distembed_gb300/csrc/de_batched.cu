@@ -104,7 +104,7 @@ KernelPick pick_kernel(int dim, bool bf16, const de_batch_shape &s, int ns = 0) 
     }
     return 0;
   };
-  k.fn = pick_staged(dim, bf16, s.pairs, s.stages, k.ctas > 1);
+  k.fn = pick_staged(dim, bf16, s.pairs, s.stages, k.ctas);
   // the column-id buffers where they fit; without them the kernel reads the ids
   // from global memory one chunk ahead
   k.stage_ids = smem_of(1) <= kStagedSmemMax ? 1 : 0;
@@ -346,7 +346,11 @@ int staged_big_graphs(const de_batch *b, const std::vector<double> &w, double to
 
 // CTAs to a cluster of the staged kernel, `from` (the shape's team_ctas) to 8,
 // whichever ends first: clusters take the big graphs, then their CTAs the others one
-// each.  STAGED_MODEL
+// each.  A minibatch of one CTA was measured at 10.7 us + 11.4 ns per CSR entry; about
+// 5 us of it, barriers and the first loads, do not shrink with the cluster.  Against
+// two-CTA clusters, two epochs of graphs of 500-50,000 vertices, dim 64, BF16: 64 graphs
+// 15.7 -> 7.8 ms from host rows to host rows, 200 graphs 22.9 -> 17.8 ms in the kernel.
+// Clusters of 16 trained the largest graph sooner but leave 40 SMs out.
 int staged_ctas(const de_batch *b, const std::vector<double> &w, double total_w, int from, int sms) {
   constexpr double kFixedUs = 5.0, kShareUs = 5.7, kEntryUs = 0.0114;
   auto cost = [&](int g, int ctas) {
@@ -388,7 +392,13 @@ int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape, const std
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || sms < 1) sms = 1;
   const bool reg = shape.kernel == DE_BATCH_REGISTER;
   if (reg) k.ctas = register_ctas(b, shape, per_sm * sms);
-  else if (k.ctas > 1) k.ctas = staged_ctas(b, w, total_w, k.ctas, per_sm * sms);
+  else if (k.ctas > 1) {
+    k.ctas = staged_ctas(b, w, total_w, k.ctas, per_sm * sms);
+    k.fn = pick_staged(b->dim, b->opt.precision == DE_PRECISION_BF16, shape.pairs, shape.stages, k.ctas);
+    // without the attribute the launch fails, and says so
+    if (cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.smem)) != cudaSuccess)
+      cudaGetLastError();
+  }
   if (k.ctas == 1) return std::min(per_sm * sms, b->n_graphs);
   // clusters of k.ctas CTAs: as many as can be resident at once (a cluster sits in one GPC)
   cudaLaunchConfig_t cfg{};

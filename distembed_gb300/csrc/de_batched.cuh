@@ -255,8 +255,8 @@ typedef void (*BatchedKernel)(BatchedArgs);
 
 // Kernel of each family for a dim, precision and shape; nullptr when none.
 BatchedKernel pick_register(int dim, bool bf16, int vpw, int warps);  // de_batched_reg.cu
-// clusters: the kernel is launched in clusters of any size (else one CTA a team)
-BatchedKernel pick_staged(int dim, bool bf16, int steps, int stages, bool clusters);  // de_batched_staged.cu
+// ctas: those of a cluster, 1 without one
+BatchedKernel pick_staged(int dim, bool bf16, int steps, int stages, int ctas);  // de_batched_staged.cu
 BatchedKernel pick_rows(int dim, bool bf16, int steps, int stages);    // de_batched_rows.cu
 
 }  // namespace batched

@@ -139,7 +139,7 @@ __device__ __forceinline__ void staged_pairs(const BatchedArgs &a, float (&acc)[
 // takes the big graphs (order[0, n_big)) as one team; when they are gone its CTAs
 // take the remaining graphs one each.  The loss of an epoch is summed from the
 // per-item losses in item order, so it does not depend on the team's make-up.
-template <int D, int NS, int S, bool kBF16, bool kClusters>
+template <int D, int NS, int S, bool kBF16, int kCtas>
 __global__ void __launch_bounds__(512, 1) staged_kernel(const BatchedArgs a) {
   using Lay = StagedLayout<D, kBF16>;
   constexpr int kRowB = Lay::kRowB, kXiB = Lay::kXiB;
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(512, 1) staged_kernel(const BatchedArgs a) {
   const unsigned char *src = kBF16 ? reinterpret_cast<const unsigned char *>(a.xb)
                                    : reinterpret_cast<const unsigned char *>(a.xm);
   const unsigned char *srcm = reinterpret_cast<const unsigned char *>(a.xm);
-  const int CT = kClusters ? cluster_ctas() : 1, rank = CT > 1 ? cluster_rank() : 0;
+  const int CT = kCtas ? kCtas : cluster_ctas(), rank = CT > 1 ? cluster_rank() : 0;
   bool coop = CT > 1;
 
   for (;;) {
@@ -329,28 +329,29 @@ __global__ void __launch_bounds__(512, 1) staged_kernel(const BatchedArgs a) {
   }
 }
 
-template <int D, bool kBF16, bool kClusters>
+template <int D, bool kBF16, int kCtas>
 BatchedKernel pick_staged_fn(int steps, int stages) {
-  if (steps == 1 && stages == 3) return staged_kernel<D, 1, 3, kBF16, kClusters>;
-  if (steps == 1 && stages == 4) return staged_kernel<D, 1, 4, kBF16, kClusters>;
-  if (steps == 2 && stages == 3) return staged_kernel<D, 2, 3, kBF16, kClusters>;
-  if (steps == 2 && stages == 4) return staged_kernel<D, 2, 4, kBF16, kClusters>;
+  if (steps == 1 && stages == 3) return staged_kernel<D, 1, 3, kBF16, kCtas>;
+  if (steps == 1 && stages == 4) return staged_kernel<D, 1, 4, kBF16, kCtas>;
+  if (steps == 2 && stages == 3) return staged_kernel<D, 2, 3, kBF16, kCtas>;
+  if (steps == 2 && stages == 4) return staged_kernel<D, 2, 4, kBF16, kCtas>;
   return nullptr;
 }
 
-template <int D>
-BatchedKernel pick_staged_dim(bool bf16, int steps, int stages, bool clusters) {
-  if (clusters) return bf16 ? pick_staged_fn<D, true, true>(steps, stages) : pick_staged_fn<D, false, true>(steps, stages);
-  return bf16 ? pick_staged_fn<D, true, false>(steps, stages) : pick_staged_fn<D, false, false>(steps, stages);
+template <int D, bool kBF16>
+BatchedKernel pick_staged_ctas(int steps, int stages, int ctas) {
+  if (ctas == 1) return pick_staged_fn<D, kBF16, 1>(steps, stages);
+  if (ctas == 2) return pick_staged_fn<D, kBF16, 2>(steps, stages);
+  return pick_staged_fn<D, kBF16, 0>(steps, stages);
 }
 
 }  // namespace
 
-BatchedKernel pick_staged(int dim, bool bf16, int steps, int stages, bool clusters) {
+BatchedKernel pick_staged(int dim, bool bf16, int steps, int stages, int ctas) {
   switch (dim) {
-    case 32: return pick_staged_dim<32>(bf16, steps, stages, clusters);
-    case 64: return pick_staged_dim<64>(bf16, steps, stages, clusters);
-    case 128: return pick_staged_dim<128>(bf16, steps, stages, clusters);
+    case 32: return bf16 ? pick_staged_ctas<32, true>(steps, stages, ctas) : pick_staged_ctas<32, false>(steps, stages, ctas);
+    case 64: return bf16 ? pick_staged_ctas<64, true>(steps, stages, ctas) : pick_staged_ctas<64, false>(steps, stages, ctas);
+    case 128: return bf16 ? pick_staged_ctas<128, true>(steps, stages, ctas) : pick_staged_ctas<128, false>(steps, stages, ctas);
   }
   return nullptr;
 }
