@@ -167,16 +167,14 @@ def spmm_roofline(alg, compulsory, step_s, peak, peak_kind):
 
 def sparse_roofline(alg, step_s, peak, peak_kind):
     """Sparse-embedding step on the DRAM side: the ncu DRAM bytes of the step's
-    captured kernels (committed summary: five attractive passes and the prune,
-    0.91 of the step's device time) over the step time; the gathered-row figure
+    kernels (committed summary) over the step time; the gathered-row figure
     beside it."""
     dram = profile_traffic("sparse_embedding_rmat20.txt")
-    return {"bound": "hbm", "kernel": "sparse step (sparse_attract_kernel<128> 5x, collect 5x, count + prune, "
-            "mirror, finalize)", "achieved": None if dram is None else dram / step_s / 1e9, "peak": peak,
+    return {"bound": "hbm", "kernel": "sparse step (sparse_attract_kernel<128> 5x, collect 5x, load, count + "
+            "prune, finalize)", "achieved": None if dram is None else dram / step_s / 1e9, "peak": peak,
             "unit": "GB/s", "frac": None if dram is None else dram / step_s / 1e9 / peak,
             "peak_source": peak_kind, "traffic": dram,
-            "basis": "ncu DRAM bytes of the captured kernels of a step (profiles/sparse_embedding_rmat20.txt; "
-                     "the uncaptured 0.09 of the step's device time not counted) / step time",
+            "basis": "ncu DRAM bytes of a step's kernels (profiles/sparse_embedding_rmat20.txt) / step time",
             "algorithmic_bytes_per_step": alg, "achieved_gathered": alg / step_s / 1e9,
             "frac_gathered": alg / step_s / 1e9 / peak,
             "note": "frac is DRAM-side; frac_gathered counts every neighbour row gathered, no reuse credited (hub "
@@ -497,7 +495,7 @@ def run_knn20k_form(args):
                        "l2": "L2-resident (10 MB FP32 embedding): latency-bound; no flush"},
             "roofline": {"bound": "l2", "achieved": achieved, "peak": l2, "unit": "GB/s", "frac": achieved / l2,
                          "peak_source": "measured here: L2-resident copy (24 MiB), 20 per event pair, best of 10",
-                         "kernel": "plain_batch_kernel<128>", "algorithmic_bytes_per_epoch": alg,
+                         "kernel": "plain_team_kernel<128, 4>", "algorithmic_bytes_per_epoch": alg,
                          "launch_us_serial": launch_us, "launches_per_epoch": batches + 1,
                          "note": "79 dependent minibatch launches per epoch of 256 rows each: one launch is a few "
                                  "microseconds of work, so launch latency and the minibatch chain bound it"},
