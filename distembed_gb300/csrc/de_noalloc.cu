@@ -63,14 +63,24 @@ struct NoAllocArgs {
 __device__ __forceinline__ float nclip(float v, float b) { return v > b ? b : (v < -b ? -b : v); }
 
 // Components of a row held by a lane: with wide loads (x 16-byte aligned, so every
-// row is) dev::Frag's, else l, l + 32, ... by 4-byte loads.
+// row is) dev::Frag's, else l, l + 32, ... by 4-byte loads.  Ordinary loads, here and
+// for the graph and the draws: the launch before may have written any of them, and a
+// load through the read-only path may be moved ahead of the wait for it.
 template <int D, bool kWide>
 __device__ __forceinline__ void nload(de::dev::Frag<D> &f, const float *row, int lane) {
-  if constexpr (kWide) {
-    de::dev::load_nc(f, row, lane);
+  constexpr int N = D / 32;
+  if constexpr (kWide && N == 2) {
+    const float2 t = reinterpret_cast<const float2 *>(row)[lane];
+    f.v[0] = t.x; f.v[1] = t.y;
+  } else if constexpr (kWide && N >= 4) {
+#pragma unroll
+    for (int h = 0; h < N / 4; ++h) {
+      const float4 t = reinterpret_cast<const float4 *>(row)[32 * h + lane];
+      f.v[4 * h] = t.x; f.v[4 * h + 1] = t.y; f.v[4 * h + 2] = t.z; f.v[4 * h + 3] = t.w;
+    }
   } else {
 #pragma unroll
-    for (int t = 0; t < D / 32; ++t) f.v[t] = __ldg(row + lane + 32 * t);
+    for (int t = 0; t < N; ++t) f.v[t] = row[lane + 32 * t];
   }
 }
 
@@ -124,8 +134,8 @@ __device__ __forceinline__ void nforces(const NoAllocArgs &a, de::dev::Frag<D> &
 // the longest chain of dependent loads.  Here a row of up to 8 W pairs is one
 // round: row pointer, column ids, rows.  Measured on the epoch of a 2,000-vertex
 // kNN graph (8 calls of 256 rows of about 14 neighbours, dim 64, 5 negatives):
-// 305 us with a warp per row and one neighbour in flight, 52 us so (6.5 us a call,
-// both launches in it).
+// 305 us with a warp per row and one neighbour in flight, 56 us so (7 us a call, both
+// launches in it).
 template <int D, int U, int W, bool kWide>
 __global__ void __launch_bounds__(W * 32) noalloc_rows_kernel(const NoAllocArgs a) {
   constexpr int N = D / 32;
@@ -135,7 +145,7 @@ __global__ void __launch_bounds__(W * 32) noalloc_rows_kernel(const NoAllocArgs 
   de::dev::pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = blockIdx.x, row = a.base + r;
-  const int e0 = __ldg(a.rowptr + row), deg = __ldg(a.rowptr + row + 1) - e0;
+  const int e0 = a.rowptr[row], deg = a.rowptr[row + 1] - e0;
   de::dev::Frag<D> xi, acc;
   nload<D, kWide>(xi, a.x + size_t(row) * D, lane);
   acc.zero();
@@ -146,12 +156,12 @@ __global__ void __launch_bounds__(W * 32) noalloc_rows_kernel(const NoAllocArgs 
   for (int q = warp; q < groups; q += W) {
     if (q < ge) {
       const int k = q * U + lane;
-      int id = lane < U && k < deg ? __ldg(a.col + e0 + k) : -1;
+      int id = lane < U && k < deg ? a.col[e0 + k] : -1;
       if (id == a.skip) id = -1;
       nforces<D, U, kWide, true>(a, acc, xi, id, want_loss, loss, lane);
     } else {
       const int k = (q - ge) * U + lane;
-      int id = lane < U && k < a.ns ? __ldg(a.negs + k) : -1;
+      int id = lane < U && k < a.ns ? a.negs[k] : -1;
       if (id >= a.n) id = -1;  // a draw equal to n contributes nothing
       nforces<D, U, kWide, false>(a, acc, xi, id, want_loss, loss, lane);
     }

@@ -124,7 +124,9 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kMinBlocks<D>)
     copy_back<D, kCopyRows>(a, lane, gw - item_ctas * kPlainWarps, (gridDim.x - item_ctas) * kPlainWarps);
     return;
   }
-  // an epoch's first minibatch reads what the launch before it writes
+  // An epoch's first minibatch reads what the launch before it writes.  The work item is
+  // loaded after the wait, and every row's address comes out of it: a read-only load
+  // whose address were known before could be moved ahead of the wait.
   if (a.first) pdl_wait();
   pdl_trigger();
   const bool has_item = gw < a.n_items;
@@ -443,7 +445,7 @@ __global__ void __launch_bounds__(256) flush_kernel(const FlushArgs a) {
   pdl_trigger();
   for (int r = gw; r < a.last_rows; r += total_w) {
     Frag<D> t;
-    load_nc(t, a.S_last + size_t(r) * D, lane);
+    load_cg(t, a.S_last + size_t(r) * D, lane);  // written by the launch before
     store<D, false>(t, a.X + size_t(a.last_base + r) * D, lane);
   }
   if (!a.compute_loss) {

@@ -67,3 +67,34 @@ def test_one_minibatch_matches_oracle(dim, n, batch, ns, shift, first):
     ulp = np.finfo(np.float32).eps * (np.abs(x0[mine]) + np.abs(want))
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want) + np.linalg.norm(ulp)
     assert abs(float(loss.item()) - want_loss) <= 1e-5 * want_loss + 1e-12
+
+
+@pytest.mark.parametrize("dim,shift", [(32, 0), (64, 4), (128, 0), (256, 4)])
+def test_calls_behind_one_another_match_calls_one_by_one(dim, shift):
+    """The same minibatch again and again, then its neighbour: each call reads rows that
+    the call queued before it writes; bitwise as with the GPU idle between the calls."""
+    import torch
+    n, batch, ns = 600, 300, 5
+    rp, col = ladder(n, 40)
+    x0 = torch.from_numpy(gg.init_embedding(n, dim, seed=dim).astype(np.float32).reshape(-1)).cuda()
+    rowptr = torch.tensor(rp, dtype=torch.int32, device="cuda")
+    cols = torch.tensor(col, dtype=torch.int32, device="cuda")
+    calls = [0] * 10 + [1, 0] * 5
+    negs = torch.tensor(np.stack([de.negatives(n, k, ns) for k in range(len(calls))]), dtype=torch.int32, device="cuda")
+    out = []
+    for idle in (True, False):
+        store = torch.zeros(n * dim + 4, dtype=torch.float32, device="cuda")
+        x = store[shift // 4: shift // 4 + n * dim]
+        x.copy_(x0)
+        loss = torch.zeros(len(calls), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        for k, j in enumerate(calls):
+            rc = de.lib().de_minibatch_noalloc(
+                n, rowptr.data_ptr(), cols.data_ptr(), dim, x.data_ptr(), j, batch, negs[k].data_ptr(), ns, batch, 1,
+                ctypes.c_float(0.02), ctypes.c_float(5.0), loss[k:].data_ptr(), torch.cuda.current_stream().cuda_stream)
+            assert rc == de.DE_OK, de.lib().de_last_error(None)
+            if idle:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        out.append((x.cpu().numpy(), loss.cpu().numpy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
