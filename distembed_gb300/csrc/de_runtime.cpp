@@ -853,7 +853,9 @@ static const double *device_view(const double *p) {
   return nullptr;
 }
 
-// Whether p is memory of the handle's GPU that 16-byte accesses can reach.
+// Whether the n x dim FP32 rows at p are memory of the handle's GPU, inside one allocation,
+// that 16-byte accesses can reach.  Others go through a copy, which reports what is wrong
+// with them.
 static bool reachable(const de_handle *h, const void *p) {
   if (reinterpret_cast<uintptr_t>(p) & 15) return false;
   cudaPointerAttributes at{};
@@ -861,7 +863,19 @@ static bool reachable(const de_handle *h, const void *p) {
     cudaGetLastError();
     return false;
   }
-  return at.type == cudaMemoryTypeDevice && at.device == h->device;
+  if (at.type != cudaMemoryTypeDevice || at.device != h->device) return false;
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr at0 = reinterpret_cast<CUdeviceptr>(p);
+  if (reinterpret_cast<decltype(&cuMemGetAddressRange)>(fn)(&base, &size, at0) != CUDA_SUCCESS) return false;
+  return at0 - base + size_t(h->n) * h->dim * sizeof(float) <= size;
 }
 
 static int copy_embeddings_f64(de_handle *h, double *host, bool to_device, float *dev = nullptr) {
@@ -1100,6 +1114,7 @@ int de_spmm_f32(de_handle *h, int32_t batch_size, float lr, float *y, int32_t on
   if (!h || !y) return DE_ERR_INVALID;
   // Memory of this GPU that the kernel's 16-byte stores can reach takes the rows
   // directly (R-MAT of 2^20 vertices, dim 128: the copy from d_y was 0.16 of 1.64 ms).
+  DE_CUDA(h, cudaSetDevice(h->device));
   if (on_device && reachable(h, y)) {
     if (int rc = spmm_run(h, batch_size, lr, y)) return rc;
     DE_CUDA(h, cudaStreamSynchronize(h->stream));
