@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, kTeamMinBlocks<D>)
   constexpr int kPairs = D >= 256 ? 4 : 8;     // pairs of a group
   constexpr int kSteps = kPairs / Lay<D>::G;
   constexpr int kGroups = 32 / kPairs;         // groups of a warp whose ids its lanes hold at once
-  __shared__ float s_acc[kTeams][W - 1][D];
+  __shared__ __align__(16) float s_acc[kTeams][W - 1][D];  // rows, 16 bytes at a time
   __shared__ float s_loss[kTeams][W - 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int team = warp / W, tw = warp % W;
