@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kRepulseThreads, 1) bf16_repulse_kernel(const 
   __shared__ __align__(8) uint64_t bar[24];
   __shared__ uint32_t tmem_holder;
   __shared__ int err;
-  __shared__ float2 negmeta[2][kChunk];  // (|n|^2, vertex id) of a chunk's negatives
+  __shared__ __align__(16) float2 negmeta[2][kChunk];  // (|n|^2, vertex id) of a chunk's negatives, read in pairs
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunks = a.kpad / kChunk;
   const int ks = blockIdx.x % a.ksplit;

@@ -8,7 +8,7 @@ import re
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-SOURCES = sorted(glob.glob(os.path.join(ROOT, "distembed_gb300", "csrc", "de_plain.cu")))
+SOURCES = sorted(glob.glob(os.path.join(ROOT, "distembed_gb300", "csrc", "*.cu")))
 DECLARED = re.compile(r"__shared__\s+(?:__align__\((\d+)\)\s+)?[\w:]+\s+(\w+)\s*\[")
 # the accesses of 16 bytes: row helpers, vector pointers, asynchronous copies
 WIDE = (r"\b(?:load|store)_lanes<[^;]*?\(\s*\w+\s*,\s*{0}\b", r"reinterpret_cast<(?:const )?(?:float4|uint4|int4|double2) \*>\(\s*&?{0}\b",
