@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -16,25 +17,29 @@ namespace de {
 
 // f(i) for i in [0, count), on host threads when count * cost_per_item is large
 // (contiguous index ranges, one per thread; f must write only what index i owns,
-// so the result does not depend on the split).
+// so the result does not depend on the split).  Where the system gives no further thread
+// the calling one takes the ranges left, so nothing is thrown at the C entry points.
 template <class F>
 void parallel_indices(int64_t count, int64_t cost_per_item, F &&f) {
   int threads = 1;
   if (count * cost_per_item >= (int64_t(1) << 18))
     threads = int(std::min<int64_t>({int64_t(std::max(1u, std::thread::hardware_concurrency())), 32, count}));
-  if (threads <= 1) {
-    for (int64_t i = 0; i < count; ++i) f(i);
-    return;
-  }
+  auto range = [&f](int64_t lo, int64_t hi) {
+    for (int64_t i = lo; i < hi; ++i) f(i);
+  };
+  if (threads <= 1) return range(0, count);
   std::vector<std::thread> pool;
+  pool.reserve(threads);
   const int64_t per = (count + threads - 1) / threads;
-  for (int t = 0; t < threads; ++t) {
-    const int64_t lo = t * per, hi = std::min(count, lo + per);
-    if (lo >= hi) break;
-    pool.emplace_back([&f, lo, hi] {
-      for (int64_t i = lo; i < hi; ++i) f(i);
-    });
+  int64_t lo = 0;
+  for (; lo < count; lo += per) {
+    try {
+      pool.emplace_back(range, lo, std::min(count, lo + per));
+    } catch (const std::system_error &) {
+      break;
+    }
   }
+  range(lo, count);
   for (auto &th : pool) th.join();
 }
 
