@@ -386,18 +386,22 @@ int staged_ctas(const de_batch *b, const std::vector<double> &w, double total_w,
 }
 
 int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape, const std::vector<double> &w, double total_w) {
+  const bool bf16 = b->opt.precision == DE_PRECISION_BF16, reg = shape.kernel == DE_BATCH_REGISTER;
   int per_sm = 0, sms = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.block, k.smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || sms < 1) sms = 1;
-  const bool reg = shape.kernel == DE_BATCH_REGISTER;
-  if (reg) k.ctas = register_ctas(b, shape, per_sm * sms);
-  else if (k.ctas > 1) {
-    k.ctas = staged_ctas(b, w, total_w, k.ctas, per_sm * sms);
-    k.fn = pick_staged(b->dim, b->opt.precision == DE_PRECISION_BF16, shape.pairs, shape.stages, k.ctas);
+  auto staged = [&](int compiled_ctas) {
+    k.fn = pick_staged(b->dim, bf16, shape.pairs, shape.stages, compiled_ctas);
     // without the attribute the launch fails, and says so
     if (cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.smem)) != cudaSuccess)
       cudaGetLastError();
+  };
+  if (reg) {
+    k.ctas = register_ctas(b, shape, per_sm * sms);
+  } else if (k.ctas > 1) {
+    k.ctas = staged_ctas(b, w, total_w, k.ctas, per_sm * sms);
+    staged(0);
   }
   if (k.ctas == 1) return std::min(per_sm * sms, b->n_graphs);
   // clusters of k.ctas CTAs: as many as can be resident at once (a cluster sits in one GPC)
@@ -417,7 +421,10 @@ int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape, const std
     cudaGetLastError();
     clusters = std::max(1, per_sm * sms / k.ctas);
   }
-  return k.ctas * std::min(clusters, b->n_graphs);
+  const int teams = k.ctas * std::min(clusters, b->n_graphs);
+  // an area a CTA, so that the cluster's size can be compiled in; fewer graphs have one each
+  if (!reg && teams <= b->n_graphs) staged(k.ctas);
+  return teams;
 }
 
 // Everything of a run except the launch: schedule, negatives, rates, team staging
@@ -464,8 +471,6 @@ int prepare_batched(de_batch *b, int epochs, int B, int ns, const double *lr, co
   if (int rc = bgrow(b, &b->d_loss, &b->loss_cap, size_t(epochs) * b->n_graphs)) return rc;
   BCUDA(b, cudaMemcpyAsync(b->d_negs, negs.data(), negs.size() * sizeof(int32_t), cudaMemcpyHostToDevice, b->stream));
   BCUDA(b, cudaMemcpyAsync(b->d_lr, lrf.data(), epochs * sizeof(float), cudaMemcpyHostToDevice, b->stream));
-  BCUDA(b, cudaMemcpyAsync(b->d_graphs, b->ginfo.data(), b->ginfo.size() * sizeof(GraphInfo), cudaMemcpyHostToDevice,
-                           b->stream));
   // graphs largest first by work (CSR entries, repulsive pairs and a fixed cost per
   // minibatch, all per epoch)
   std::vector<double> w(b->n_graphs);
@@ -477,13 +482,22 @@ int prepare_batched(de_batch *b, int epochs, int B, int ns, const double *lr, co
   std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) { return w[x] > w[y]; });
   const int teams = teams_for(b, k, shape, w, total_w);
   b->n_big = k.ctas > 1 && shape.kernel != DE_BATCH_REGISTER ? staged_big_graphs(b, w, total_w, teams) : 0;
+  for (int g = 0; g < b->n_graphs; ++g) b->ginfo[g].area = teams > b->n_graphs ? g : -1;
+  BCUDA(b, cudaMemcpyAsync(b->d_graphs, b->ginfo.data(), b->ginfo.size() * sizeof(GraphInfo), cudaMemcpyHostToDevice,
+                           b->stream));
   BCUDA(b, cudaMemcpyAsync(b->d_order, b->order.data(), b->order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                            b->stream));
   BCUDA(b, cudaStreamSynchronize(b->stream));  // the host vectors go away on return
-  if (int rc = bgrow(b, &b->d_stage, &b->stage_cap, size_t(teams) * B * b->dim)) return rc;
-  if (int rc = bgrow(b, &b->d_slots, &b->slots_cap, size_t(teams) * b->max_slots * b->dim)) return rc;
-  if (int rc = bgrow(b, &b->d_item_loss, &b->item_loss_cap, size_t(teams) * b->max_batch_items)) return rc;
-  if (int rc = bgrow(b, &b->d_cluster_slot, &b->cluster_slot_cap, size_t(teams / std::max(k.ctas, 1) + 1)))
+  // Staging areas, of the rows of the largest minibatch.  A cluster of the register kernel
+  // has one.  In the staged kernel every CTA may come to train a graph alone, but no more
+  // areas are in use than there are graphs.
+  const int clusters = teams / std::max(k.ctas, 1);
+  const int areas = shape.kernel == DE_BATCH_REGISTER ? clusters : std::min(teams, b->n_graphs);
+  const int rows = int(std::min<int64_t>(B, *std::max_element(b->n.begin(), b->n.end())));
+  if (int rc = bgrow(b, &b->d_stage, &b->stage_cap, size_t(areas) * rows * b->dim)) return rc;
+  if (int rc = bgrow(b, &b->d_slots, &b->slots_cap, size_t(areas) * b->max_slots * b->dim)) return rc;
+  if (int rc = bgrow(b, &b->d_item_loss, &b->item_loss_cap, size_t(areas) * b->max_batch_items)) return rc;
+  if (int rc = bgrow(b, &b->d_cluster_slot, &b->cluster_slot_cap, size_t(clusters + 1)))
     return rc;
   BatchedArgs &a = b->args;
   a = BatchedArgs{};
@@ -508,6 +522,7 @@ int prepare_batched(de_batch *b, int epochs, int B, int ns, const double *lr, co
   a.loss_from = b->loss_mode == DE_LOSS_LAST_EPOCH ? epochs - 1 : 0;
   a.bound = float(b->opt.max_bound);
   a.stage = b->d_stage;
+  a.stage_rows = rows;
   a.slots = b->d_slots;
   a.slot_stride = b->max_slots;
   a.loss = b->d_loss;

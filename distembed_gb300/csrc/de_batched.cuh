@@ -24,7 +24,7 @@ struct GraphInfo {
   int64_t batch_off; // first minibatch of the graph in the per-minibatch tables
   int64_t neg_off;   // first negative of the graph (per run: [epochs, batches, ns])
   int32_t n, batches, last_batch_size;
-  int32_t pad;
+  int32_t area;      // staged kernel: the graph's staging area where it has one of its own, else -1
 };
 
 struct SplitRow {
@@ -47,21 +47,22 @@ struct BatchedArgs {
   const float *lr;           // [epochs]
   int32_t epochs, batch, ns, quirks, compute_loss;
   float bound;
-  float *stage;              // [teams, batch, dim] staged updates
-  float *slots;              // [teams, max slots, dim] partials of split rows
-  int32_t slot_stride;       // slots per team
+  float *stage;              // [areas, stage_rows, dim] staged updates
+  int32_t stage_rows;        // rows of the largest minibatch
+  float *slots;              // [areas, max slots, dim] partials of split rows
+  int32_t slot_stride;       // slots per area
   double *loss;              // [n_graphs, epochs]
   float near_r;              // BF16 form: pairs closer than this are recomputed in FP32
   long long *trace;          // nullable: per graph {start ns, end ns, team}
   int32_t cap;               // staged kernel: CSR entries per chunk (<= 32)
   int32_t *err;              // staged kernel: set when a bounded wait gives up
-  // staged kernel with two-CTA teams: the first n_big graphs of `order` are trained
-  // by both CTAs of a cluster together (next_big counts them out), the rest by
-  // single CTAs (next_graph counts from order[n_big])
+  // staged kernel with teams of several CTAs: the first n_big graphs of `order` are
+  // trained by a cluster's CTAs together (next_big counts them out), the rest by single
+  // CTAs (next_graph counts from order[n_big])
   int32_t n_big;
   int32_t *next_big;
   int32_t *cluster_slot;     // [clusters] graph handed from CTA rank 0 to the others
-  float *item_loss;          // [teams, max items of a minibatch] loss of every work item
+  float *item_loss;          // [areas, max items of a minibatch] loss of every work item
   int32_t item_stride;
   int32_t loss_from;         // epochs e >= loss_from (of this run) compute their loss; the others write 0
   int32_t stage_ids;         // staged kernel: 1 = a round's column ids are prefetched into shared memory
@@ -255,7 +256,7 @@ typedef void (*BatchedKernel)(BatchedArgs);
 
 // Kernel of each family for a dim, precision and shape; nullptr when none.
 BatchedKernel pick_register(int dim, bool bf16, int vpw, int warps);  // de_batched_reg.cu
-// ctas: those of a cluster, 1 without one
+// ctas: those of a cluster where its size is compiled in, 1 without one, 0: read at run time
 BatchedKernel pick_staged(int dim, bool bf16, int steps, int stages, int ctas);  // de_batched_staged.cu
 BatchedKernel pick_rows(int dim, bool bf16, int steps, int stages);    // de_batched_rows.cu
 

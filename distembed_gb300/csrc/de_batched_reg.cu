@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
     if (nct > 1) cluster_sync();
     else __syncthreads();
   };
-  float *stage = a.stage + size_t(team) * a.batch * D;
+  float *stage = a.stage + size_t(team) * a.stage_rows * D;
   float *slots = a.slots + size_t(team) * a.slot_stride * D;
   float *item_loss = a.item_loss + size_t(team) * a.item_stride;
   const int skip_last = a.quirks;

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(512, 1) staged_rows_kernel(const BatchedArgs a
   const uint32_t ring_s = dev::smem_u32(ring), neg_s = dev::smem_u32(negrows);
   __shared__ int sh_graph;
   __shared__ double sh_loss[16];
-  float *stage = a.stage + size_t(blockIdx.x) * a.batch * D;
+  float *stage = a.stage + size_t(blockIdx.x) * a.stage_rows * D;
   float *slots = a.slots + size_t(blockIdx.x) * a.slot_stride * D;
   const unsigned char *src = kBF16 ? reinterpret_cast<const unsigned char *>(a.xb)
                                    : reinterpret_cast<const unsigned char *>(a.xm);

@@ -134,11 +134,13 @@ __device__ __forceinline__ void staged_pairs(const BatchedArgs &a, float (&acc)[
 
 
 // A team is one CTA or, launched in clusters of CT CTAs, those of a cluster working on
-// one graph: team warp tw = rank * W + warp of TW = nct * W, one shared staging area
-// (that of rank 0), barriers across the cluster.  With CT > 1 a cluster first
-// takes the big graphs (order[0, n_big)) as one team; when they are gone its CTAs
-// take the remaining graphs one each.  The loss of an epoch is summed from the
-// per-item losses in item order, so it does not depend on the team's make-up.
+// one graph: team warp tw = rank * W + warp of TW = nct * W, one shared staging area,
+// barriers across the cluster.  With CT > 1 a cluster first takes the big graphs
+// (order[0, n_big)) as one team; when they are gone its CTAs take the remaining graphs
+// one each.  The loss of an epoch is summed from the per-item losses in item order, so it
+// does not depend on the team's make-up.  kCtas = 0: CT is read at run time, and a graph
+// may have a staging area of its own (GraphInfo::area); else the area is the one of the
+// team's first CTA.
 template <int D, int NS, int S, bool kBF16, int kCtas>
 __global__ void __launch_bounds__(512, 1) staged_kernel(const BatchedArgs a) {
   using Lay = StagedLayout<D, kBF16>;
@@ -188,10 +190,11 @@ __global__ void __launch_bounds__(512, 1) staged_kernel(const BatchedArgs a) {
     }
     const int nct = coop ? CT : 1, trank = coop ? rank : 0;
     const int tw = trank * W + warp, TW = nct * W;
-    const int team_blk = blockIdx.x - trank;
-    float *stage = a.stage + size_t(team_blk) * a.batch * D;
-    float *slots = a.slots + size_t(team_blk) * a.slot_stride * D;
-    float *item_loss = a.item_loss + size_t(team_blk) * a.item_stride;
+    int area = blockIdx.x - trank;
+    if (kCtas == 0 && a.graphs[g].area >= 0) area = a.graphs[g].area;
+    float *stage = a.stage + size_t(area) * a.stage_rows * D;
+    float *slots = a.slots + size_t(area) * a.slot_stride * D;
+    float *item_loss = a.item_loss + size_t(area) * a.item_stride;
     auto team_sync = [&]() {
       if (nct > 1) cluster_sync();
       else __syncthreads();
