@@ -345,6 +345,10 @@ template <int D, bool kBF16>
 BatchedKernel pick_staged_ctas(int steps, int stages, int ctas) {
   if (ctas == 1) return pick_staged_fn<D, kBF16, 1>(steps, stages);
   if (ctas == 2) return pick_staged_fn<D, kBF16, 2>(steps, stages);
+  // four compiled in pay at dim 128 alone (1,000 graphs, two steps: 2-4 % against the size
+  // read at run time; at dim 32 and 64 they cost 1-4 %)
+  if constexpr (D == 128)
+    if (ctas == 4) return pick_staged_fn<D, kBF16, 4>(steps, stages);
   return pick_staged_fn<D, kBF16, 0>(steps, stages);
 }
 
