@@ -70,7 +70,7 @@ KernelPick pick_kernel(int dim, bool bf16, const de_batch_shape &s, int ns = 0) 
   k.ctas = s.team_ctas > 1 ? s.team_ctas : 1;
   if (s.kernel == DE_BATCH_REGISTER) {
     if (s.edge_cap < 1 || s.edge_cap > 4096) return k;
-    k.fn = pick_register(dim, bf16, s.vertices_per_warp, s.team_warps);
+    k.fn = pick_register(dim, bf16, s.vertices_per_warp, s.team_warps, false);
     k.block = 32 * s.team_warps;
     return k;
   }
@@ -399,6 +399,7 @@ int teams_for(de_batch *b, KernelPick &k, const de_batch_shape &shape, const std
   };
   if (reg) {
     k.ctas = register_ctas(b, shape, per_sm * sms);
+    if (k.ctas > 1) k.fn = pick_register(b->dim, bf16, shape.vertices_per_warp, shape.team_warps, true);
   } else if (k.ctas > 1) {
     k.ctas = staged_ctas(b, w, total_w, k.ctas, per_sm * sms);
     staged(0);

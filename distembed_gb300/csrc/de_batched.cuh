@@ -255,7 +255,7 @@ struct RowsLayout {
 typedef void (*BatchedKernel)(BatchedArgs);
 
 // Kernel of each family for a dim, precision and shape; nullptr when none.
-BatchedKernel pick_register(int dim, bool bf16, int vpw, int warps);  // de_batched_reg.cu
+BatchedKernel pick_register(int dim, bool bf16, int vpw, int warps, bool cluster);  // de_batched_reg.cu
 // ctas: those of a cluster where its size is compiled in, 1 without one, 0: read at run time
 BatchedKernel pick_staged(int dim, bool bf16, int steps, int stages, int ctas);  // de_batched_staged.cu
 BatchedKernel pick_rows(int dim, bool bf16, int steps, int stages);    // de_batched_rows.cu

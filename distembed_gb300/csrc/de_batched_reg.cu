@@ -67,22 +67,34 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 
-// Rows in flight per group: eight where a lane's share of a row is small.
-template <int D, int VPW>
-constexpr int kInFlight = Row<D, VPW>::L >= 8 && Row<D, VPW>::P <= 4 ? 8 : 4;
+// Rows in flight per group.  Eight take more registers, and at most shapes a resident CTA
+// with them (dim 32, vertices_per_warp 4, 8 warps, 1,000 graphs: 2.52 ms against 1.55 with
+// four).  They pay where they do not and a cluster's short chains are what bounds a
+// minibatch: dim 32, FP32, 24 and 64 graphs on clusters of eight 4-7 % (BF16 loses 4 %).
+template <int D, int VPW, int WARPS, bool kBF16, bool kCluster>
+constexpr int kInFlight = kCluster && !kBF16 && D == 32 && VPW == 4 && (WARPS == 8 || WARPS == 16) ? 8 : 4;
 
-// Forces of up to kInFlight rows named by lanes [k, k + kInFlight) of the group (ids < 0: none),
+// Resident CTAs the registers are held to where the compiler alone takes one too many for
+// the fourth (0: its own choice).  400 graphs, dim 64: 16.0 ms at 160 registers, 14.1 before.
+template <int D, int VPW, int WARPS>
+constexpr int kMinCtas = D == 64 && VPW == 2 && WARPS == 4 ? 4 : 0;
+
+// Whether a chunk's column ids are loaded a chunk ahead.  At dim 128, FP32, a row to a
+// warp of sixteen the registers for it are not there: 400 graphs 9.6 ms so, 8.5 without.
+template <int D, int VPW, int WARPS, bool kBF16, bool kCluster>
+constexpr bool kIdsAhead = kCluster || kBF16 || D != 128 || VPW != 1 || WARPS != 16;
+
+// Forces of up to U rows named by lanes [k, k + U) of the group (ids < 0: none),
 // all groups of the warp in step (the caller keeps the warp converged).  xi is the
 // row's FP32 master value.  In the BF16 form the rows are read as BF16; a pair
 // whose squared distance from those reads is below a.near_r is read again from
 // the FP32 master and recomputed, so that the rounding of the copy does not bias
 // close pairs (their distance is then comparable with the BF16 rounding step).
-template <int D, int VPW, bool kBF16, bool kAttract>
+template <int D, int VPW, int U, bool kBF16, bool kAttract>
 __device__ __forceinline__ void group_forces(const BatchedArgs &a, Row<D, VPW> &acc, const Row<D, VPW> &xi,
                                              int64_t voff, int ids, int k, int gbase, int gl, float lr,
                                              float &loss, bool want) {
   constexpr int L = Row<D, VPW>::L, P = Row<D, VPW>::P;
-  constexpr int U = kInFlight<D, VPW>;
   Row<D, VPW> xn[U];
   int nid[U];
   float r[U];
@@ -137,18 +149,20 @@ __device__ __forceinline__ void group_forces(const BatchedArgs &a, Row<D, VPW> &
   }
 }
 
-template <int D, int VPW, int WARPS, bool kBF16>
-__global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a) {
-  constexpr int L = Row<D, VPW>::L, P = Row<D, VPW>::P, U = kInFlight<D, VPW>;
+// kCluster: a team is the CTAs of the cluster that the kernel is launched in, else one CTA
+// (a kernel of its own: the cluster's run-time size takes up to 45 registers).
+template <int D, int VPW, int WARPS, bool kBF16, bool kCluster>
+__global__ void __launch_bounds__(WARPS * 32, kMinCtas<D, VPW, WARPS>) batched_kernel(const BatchedArgs a) {
+  constexpr int L = Row<D, VPW>::L, P = Row<D, VPW>::P, U = kInFlight<D, VPW, WARPS, kBF16, kCluster>;
   static_assert(P % 2 == 0, "components per lane must be even");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane / L, gl = lane % L, gbase = grp * L;
   __shared__ int sh_graph;
   // team: nct CTAs (those of the cluster), this one its rank-th
-  const int nct = cluster_ctas(), rank = nct > 1 ? cluster_rank() : 0;
+  const int nct = kCluster ? cluster_ctas() : 1, rank = kCluster ? cluster_rank() : 0;
   const int team = blockIdx.x / nct, tw = rank * WARPS + warp, TW = nct * WARPS;
   auto team_sync = [&]() {
-    if (nct > 1) cluster_sync();
+    if (kCluster) cluster_sync();
     else __syncthreads();
   };
   float *stage = a.stage + size_t(team) * a.stage_rows * D;
@@ -161,11 +175,11 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
     if (threadIdx.x == 0 && rank == 0) {
       const int i = atomicAdd(a.next_graph, 1);
       g = i < a.n_graphs ? a.order[i] : -1;
-      if (nct > 1) *reinterpret_cast<volatile int *>(a.cluster_slot + team) = g;
+      if (kCluster) *reinterpret_cast<volatile int *>(a.cluster_slot + team) = g;
       else sh_graph = g;
     }
     team_sync();
-    g = nct > 1 ? __ldcg(a.cluster_slot + team) : sh_graph;
+    g = kCluster ? __ldcg(a.cluster_slot + team) : sh_graph;
     team_sync();  // the slot is rewritten only after every thread has read it
     if (g < 0) return;
     if (a.trace && threadIdx.x == 0 && rank == 0) {
@@ -205,12 +219,14 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
           int maxcnt = cnt;
 #pragma unroll
           for (int m = 16; m >= L; m >>= 1) maxcnt = max(maxcnt, __shfl_xor_sync(kAll, maxcnt, m));
-          int next = gl < cnt ? __ldg(cols + gl) : -1;
+          constexpr bool kAhead = kIdsAhead<D, VPW, WARPS, kBF16, kCluster>;
+          int next = kAhead && gl < cnt ? __ldg(cols + gl) : -1;
           for (int c0 = 0; c0 < maxcnt; c0 += L) {
+            if constexpr (!kAhead) next = gl < cnt - c0 ? __ldg(cols + c0 + gl) : -1;
             const int ids = next == skip ? -1 : next;
-            next = gl < cnt - c0 - L ? __ldg(cols + c0 + L + gl) : -1;  // the next chunk's ids, a chunk ahead
+            if constexpr (kAhead) next = gl < cnt - c0 - L ? __ldg(cols + c0 + L + gl) : -1;
             for (int k = 0; k < L && c0 + k < maxcnt; k += U)
-              group_forces<D, VPW, kBF16, true>(a, acc, xi, G.voff, ids, k, gbase, gl, lr, loss, want);
+              group_forces<D, VPW, U, kBF16, true>(a, acc, xi, G.voff, ids, k, gbase, gl, lr, loss, want);
           }
           const bool repulse = has && it.part == 0 && it.row < rep_rows;
           const bool any_rep = __any_sync(kAll, repulse);
@@ -221,7 +237,7 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
               if (ids >= G.n) ids = -1;  // a draw equal to n contributes nothing
             }
             for (int k = 0; k < L && k0 + k < a.ns; k += U)
-              group_forces<D, VPW, kBF16, false>(a, acc, xi, G.voff, ids, k, gbase, gl, lr, loss, want);
+              group_forces<D, VPW, U, kBF16, false>(a, acc, xi, G.voff, ids, k, gbase, gl, lr, loss, want);
           }
           if (has) {
             float *dst = it.nparts > 1 ? slots + size_t(it.first_slot + it.part) * D : stage + size_t(it.row) * D;
@@ -253,36 +269,41 @@ __global__ void __launch_bounds__(WARPS * 32) batched_kernel(const BatchedArgs a
 template <int D, int V>
 constexpr bool kShapeOk = (D / (32 / V)) % 2 == 0;
 
+template <int D, bool kBF16, int V, int W>
+BatchedKernel pick_team(bool cluster) {
+  return cluster ? batched_kernel<D, V, W, kBF16, true> : batched_kernel<D, V, W, kBF16, false>;
+}
+
 template <int D, bool kBF16, int V>
-BatchedKernel pick_warps(int warps) {
+BatchedKernel pick_warps(int warps, bool cluster) {
   if constexpr (kShapeOk<D, V>) {
     switch (warps) {
-      case 4: return batched_kernel<D, V, 4, kBF16>;
-      case 8: return batched_kernel<D, V, 8, kBF16>;
-      case 16: return batched_kernel<D, V, 16, kBF16>;
-      case 32: return batched_kernel<D, V, 32, kBF16>;
+      case 4: return pick_team<D, kBF16, V, 4>(cluster);
+      case 8: return pick_team<D, kBF16, V, 8>(cluster);
+      case 16: return pick_team<D, kBF16, V, 16>(cluster);
+      case 32: return pick_team<D, kBF16, V, 32>(cluster);
     }
   }
   return nullptr;
 }
 
 template <int D, bool kBF16>
-BatchedKernel pick(int vpw, int warps) {
+BatchedKernel pick(int vpw, int warps, bool cluster) {
   switch (vpw) {
-    case 1: return pick_warps<D, kBF16, 1>(warps);
-    case 2: return pick_warps<D, kBF16, 2>(warps);
-    case 4: return pick_warps<D, kBF16, 4>(warps);
+    case 1: return pick_warps<D, kBF16, 1>(warps, cluster);
+    case 2: return pick_warps<D, kBF16, 2>(warps, cluster);
+    case 4: return pick_warps<D, kBF16, 4>(warps, cluster);
   }
   return nullptr;
 }
 
 }  // namespace
 
-BatchedKernel pick_register(int dim, bool bf16, int vpw, int warps) {
+BatchedKernel pick_register(int dim, bool bf16, int vpw, int warps, bool cluster) {
   switch (dim) {
-    case 32: return bf16 ? pick<32, true>(vpw, warps) : pick<32, false>(vpw, warps);
-    case 64: return bf16 ? pick<64, true>(vpw, warps) : pick<64, false>(vpw, warps);
-    case 128: return bf16 ? pick<128, true>(vpw, warps) : pick<128, false>(vpw, warps);
+    case 32: return bf16 ? pick<32, true>(vpw, warps, cluster) : pick<32, false>(vpw, warps, cluster);
+    case 64: return bf16 ? pick<64, true>(vpw, warps, cluster) : pick<64, false>(vpw, warps, cluster);
+    case 128: return bf16 ? pick<128, true>(vpw, warps, cluster) : pick<128, false>(vpw, warps, cluster);
   }
   return nullptr;
 }
