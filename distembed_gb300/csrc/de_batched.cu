@@ -304,18 +304,19 @@ int build_batched_schedule(de_batch *b, int B, int cap) {
 
 // CTAs to a team of the register kernel: 1, 2, 4 or 8 (a portable cluster), whichever
 // ends first when the graphs go largest first to the teams that fit the GPU at once.
-// A minibatch costs a team its barriers and update and, per round of its warps over
-// the minibatch's items, the chain of loads of the longest row; the two constants
-// only have to rank the sizes (256 rows a minibatch, vertices_per_warp 4, 8 warps:
-// about 57 us at one CTA, 8 rounds, 10 us at eight).  Measured, ms for two epochs at
-// 1 / 2 / 4 / 8 CTAs a team: 24 graphs of 500-5,000, dim 32: 2.03 / 1.23 / 0.79 /
-// 0.58; 64 of 500-50,000, dim 64: 30.1 / 17.3 / 12.3 / 8.6; 256 of 500-10,000, dim
-// 64: 6.5 / 4.2 / 3.0 / 4.3; dim 32, 512 rows: 4.7 / 2.6 / 3.1 / 4.9.  The rule took
-// the smallest of each.
+// A minibatch costs a team a round of its warps over the minibatch's items, again and
+// again, and its barriers, update and first loads, which more CTAs do not shorten: about
+// three rounds' time.  Measured at 1 / 2 / 4 / 8 CTAs a team and 12 shapes of 4 to 32
+// warps, dim 32 to 128, FP32 and BF16, on 3 to 1,000 graphs (384 settings): the rule's
+// size is 0.5 % from the best on average, 15 % at most (0.6 rounds, which an earlier rule
+// took from shapes of 8 warps alone: 2.6 % and 47 %, the wide teams among many graphs).
+// For instance ms for two epochs, dim 64, FP32: 400 graphs, vertices_per_warp 2, 8 warps
+// 7.92 / 4.48 / 4.56 / 5.87, 2 and 16 warps 4.70 / 4.89 / 6.94 / 13.3, 4 and 32 warps 4.63
+// / 6.43 / 12.1 / 29.1; 24 graphs, 4 and 8 warps 2.71 / 1.60 / 1.03 / 0.76.
 int register_ctas(const de_batch *b, const de_batch_shape &s, int resident) {
-  constexpr double kFixedUs = 4.0, kRoundUs = 6.5;
+  constexpr double kFixedRounds = 3.0;
   int best = 1;
-  double best_us = -1;
+  double best_end = -1;
   for (int ctas : {1, 2, 4, 8}) {
     const int per_round = ctas * s.team_warps * s.vertices_per_warp;
     const int teams = std::min(resident / ctas, b->n_graphs);
@@ -326,12 +327,12 @@ int register_ctas(const de_batch *b, const de_batch_shape &s, int resident) {
     for (int g : b->order) {
       const GraphInfo &G = b->ginfo[g];
       const double items = double(b->graph_items[g]) / G.batches;
-      const double us = busy.top() + G.batches * (kFixedUs + kRoundUs * std::ceil(items / per_round));
+      const double at = busy.top() + G.batches * (kFixedRounds + std::ceil(items / per_round));
       busy.pop();
-      busy.push(us);
-      end = std::max(end, us);
+      busy.push(at);
+      end = std::max(end, at);
     }
-    if (best_us < 0 || end < best_us) best = ctas, best_us = end;
+    if (best_end < 0 || end < best_end) best = ctas, best_end = end;
   }
   return best;
 }
