@@ -115,6 +115,10 @@ struct PlainBatchArgs {
 };
 
 constexpr int kStageSlots = 4;   // staging buffers of the FP32 plain form, a ring over the minibatches
+// Rows of a minibatch's buffers (a minibatch may be larger than the graph), and the
+// staging buffers that an FP32 run of `batches` minibatches uses.
+inline size_t batch_rows(int64_t n, int64_t batch) { return size_t(std::min(batch, n)); }
+inline size_t stage_slots(int64_t batches) { return size_t(std::min<int64_t>(batches, kStageSlots)); }
 constexpr int kStageNegMax = 8;  // negatives per minibatch the shared-memory staging takes
 
 struct FlushArgs {

@@ -480,10 +480,6 @@ PlainBatchArgs plain_args(const de_handle *h, int ns) {
 // the edge cap asks for one warp a work item of that size.
 bool item_teams(const de_handle *h, const PlainBatchArgs &a) { return h->opt.edge_cap <= 0 && !a.stage_negs; }
 
-// Rows of a staging buffer, and how many an epoch of the schedule uses.
-size_t stage_rows(const Schedule &s, int64_t n) { return size_t(std::min<int64_t>(s.batch, n)); }
-size_t stage_slots(const Schedule &s) { return size_t(std::min(s.batches, kStageSlots)); }
-
 // Epochs of one minibatch whose per-item losses are kept at once.
 int loss_epochs(const de_handle *h, int epochs) {
   return int(std::min<int64_t>(epochs, std::max<int64_t>(1, kEpochLossItems / std::max<int64_t>(1, h->sched.n_items))));
@@ -530,7 +526,7 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
   cudaError_t err = cudaSuccess;
   for (int j = 0; j < s.batches && err == cudaSuccess; ++j) {
     PlainBatchArgs a = plain_args(h, ns);
-    const size_t slice = stage_rows(s, h->n) * h->dim;
+    const size_t slice = batch_rows(h->n, s.batch) * h->dim;
     a.S_cur = h->d_stage + slice * (j % kStageSlots);
     a.S_prev = h->d_stage + slice * ((j + kStageSlots - 1) % kStageSlots);
     a.S_prev2 = h->d_stage + slice * ((j + kStageSlots - 2) % kStageSlots);
@@ -551,7 +547,7 @@ cudaError_t enqueue_epoch_plain(de_handle *h, int ns, cudaStream_t st, cudaEvent
   if (err == cudaSuccess) {
     FlushArgs f{};
     f.X = h->d_x;
-    f.S_last = h->d_stage + stage_rows(s, h->n) * h->dim * ((s.batches - 1) % kStageSlots);
+    f.S_last = h->d_stage + batch_rows(h->n, s.batch) * h->dim * ((s.batches - 1) % kStageSlots);
     f.last_base = int32_t(int64_t(s.batches - 1) * s.batch);
     f.last_rows = s.last_batch_size;
     f.loss_partial = h->d_loss_partial;
@@ -956,7 +952,7 @@ static int prepare_run(de_handle *h, int32_t first_epoch, int32_t epochs, int32_
   bool moved = false;
   int rc = DE_OK;
   const bool bf16 = h->opt.precision == DE_PRECISION_BF16;
-  if (!bf16 && (rc = grow(h, &h->d_stage, &h->stage_cap, stage_slots(s) * stage_rows(s, h->n) * h->dim, &moved)) != DE_OK) return rc;
+  if (!bf16 && (rc = grow(h, &h->d_stage, &h->stage_cap, stage_slots(s.batches) * batch_rows(h->n, s.batch) * h->dim, &moved)) != DE_OK) return rc;
   if (bf16 && (rc = ensure_bf16_buffers(h, ns, &moved)) != DE_OK) return rc;
   bool counters_moved = false;
   const int keep = !bf16 && s.batches == 1 && h->opt.compute_loss ? loss_epochs(h, epochs) : 1;
@@ -976,9 +972,11 @@ static int prepare_run(de_handle *h, int32_t first_epoch, int32_t epochs, int32_
   if (size_t(epochs) > h->lr_cap || !h->d_lr)
     if ((rc = grow(h, &h->d_lr, &h->lr_cap, ecap, &moved))) return rc;
   const size_t nneg = size_t(epochs) * s.batches * std::max(ns, 1);
+  // room for longer runs, but none in an arena: a served job makes one run, and no more
+  // than that is reserved for it
+  const size_t negs_room = h->hooks.dalloc ? nneg : std::max(nneg, ecap * s.batches * std::max(ns, 1));
   if (nneg > h->negs_cap || !h->d_negs)
-    if ((rc = grow(h, &h->d_negs, &h->negs_cap, std::max(nneg, ecap * s.batches * std::max(ns, 1)), &moved)))
-      return rc;
+    if ((rc = grow(h, &h->d_negs, &h->negs_cap, negs_room, &moved))) return rc;
   if (moved) drop_graph(h);
 
   // Host side of the upload: wait until the previous call's copies have read

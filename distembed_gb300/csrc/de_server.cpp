@@ -114,32 +114,36 @@ struct Job {
 // buffers: graph, embedding, work lists, staging, per-call arrays, BF16 form).
 int64_t job_bytes(const de_job_spec &s) {
   const int64_t n = s.n, nnz = s.nnz, D = s.dim, B = s.batch_size;
-  const int64_t batches = (n + B - 1) / B;
-  constexpr int64_t cap = 32;
-  // work items: one per row plus one per further cap-sized piece of a long row
-  int64_t items = 0, max_items = 0;
+  const int64_t batches = (n + B - 1) / B, rows = int64_t(de::batch_rows(n, B));
+  constexpr int64_t cap = de::kMaxEdgeCap;
+  // work items: one per row, or one per cap-sized piece of a long row; such pieces, and
+  // their groups, have partial slots and no more counters than that
+  int64_t items = 0, max_parts = 0;
   for (int64_t j = 0; j < batches; ++j) {
-    int64_t bi = 0;
+    int64_t parts = 0;
     const int64_t r1 = std::min(n, (j + 1) * B);
     for (int64_t r = j * B; r < r1; ++r) {
-      const int64_t deg = s.rowptr[r + 1] - s.rowptr[r];
-      bi += deg <= cap ? 1 : (deg + cap - 1) / cap + (deg + cap - 1) / cap / 16 + 1;
+      const int64_t deg = s.rowptr[r + 1] - s.rowptr[r], np = (deg + cap - 1) / cap;
+      items += deg <= cap ? 1 : np;
+      if (deg > cap) parts += np + (np > de::kCombineGroup ? (np + de::kCombineGroup - 1) / de::kCombineGroup : 0);
     }
-    items += bi;
-    max_items = std::max(max_items, bi);
+    max_parts = std::max(max_parts, parts);
   }
   int64_t b = 4 * (n + 1) + 4 * std::max<int64_t>(nnz, 1) + 4 * n * D;  // CSR, embedding
   b += 32 * items;                                                      // work items
-  b += de::kStageSlots * B * D * 4 + max_items * D * 4 + max_items * 4;               // staging, partial slots, counters
-  // per-item loss partials, of several epochs when the minibatch is the whole graph
+  b += max_parts * D * 4 + max_parts * 4;                               // partial slots, counters
+  // per-item loss partials and their sums, of several epochs when the minibatch is the whole graph
   b += 8 * (batches > 1 ? items : std::max(items, std::min(items * s.epochs, de::kEpochLossItems)));
-  b += int64_t(s.epochs) * (batches * s.ns * 4 + 16);                   // negatives, rates, losses
+  if (batches == 1) b += 8 * (s.epochs + de::kEpochLossItems / de::kFlushChunk);
+  b += int64_t(s.epochs) * (batches * std::max(s.ns, 1) * 4 + 16);      // negatives, rates, losses
   b += 8 * 2048;                                                        // small fixed buffers
   if (s.precision == DE_PRECISION_BF16) {
     const int64_t kpad = std::max<int64_t>(64, (s.ns + 63) / 64 * 64);
-    const int64_t parts = de::bf16_ksplit(std::min(n, B), kpad);
+    const int64_t parts = de::bf16_ksplit(rows, kpad);
     b += 2 * n * D + 8 * n + (1 + parts) * B * D * 4 + parts * B * 8;  // + update rows and their losses
     b += 2 * kpad * D * 2 + kpad * 8 + B * 32 * 4;
+  } else {
+    b += int64_t(de::stage_slots(batches)) * rows * D * 4;             // staging
   }
   return b + b / 16 + (1 << 20);  // allocator rounding and slack
 }
