@@ -183,10 +183,10 @@ struct BF16BatchArgs {
   const int32_t *epoch;     // device [2]
   float *P;                 // partial slots of split rows
   int32_t *counters;
-  float *abuf;              // [B, dim] attractive update of the minibatch (lr applied)
-  float *rbuf;              // [ksplit, B, dim] repulsive (GEMM) update of the minibatch (lr applied), in parts
-  double *rloss;            // [ksplit, B] its loss, likewise
-  int32_t ksplit, rstride;  // CTAs that share a tile's negatives; rows of a part (B)
+  float *abuf;              // [rows, dim] attractive update of the minibatch (lr applied)
+  float *rbuf;              // [ksplit, rstride, dim] repulsive (GEMM) update of the minibatch (lr applied), in parts
+  double *rloss;            // [ksplit, rstride] its loss, likewise
+  int32_t ksplit, rstride;  // CTAs that share a tile's negatives; rows of a part (the largest minibatch's)
   __nv_bfloat16 *nb;        // [kpad, dim] gathered negatives
   float *nn;                // [kpad] squared norms of the gathered negatives
   int32_t *nid;             // [kpad] vertex id of each negative, -1 = none

@@ -381,7 +381,7 @@ cudaError_t enqueue_epoch_bf16(de_handle *h, int ns, cudaStream_t st, cudaEvent_
     a.rbuf = h->d_rbuf;
     a.rloss = h->d_rloss;
     a.ksplit = h->ksplit;
-    a.rstride = s.batch;
+    a.rstride = int32_t(batch_rows(h->n, s.batch));
     a.nb = h->d_nb;
     a.nn = h->d_nn;
     a.nid = h->d_nid;
@@ -415,14 +415,15 @@ int ensure_bf16_buffers(de_handle *h, int ns, bool *moved) {
   const Schedule &s = h->sched;
   const int kpad = std::max(64, (ns + 63) / 64 * 64);
   if (kpad > 1024) return fail(h, DE_ERR_UNSUPPORTED, "the BF16 form takes at most 1024 negatives per minibatch");
-  const int ksplit = bf16_ksplit(std::min<int64_t>(s.batch, h->n), kpad);
+  const size_t rows = batch_rows(h->n, s.batch);
+  const int ksplit = bf16_ksplit(int64_t(rows), kpad);
   bool m = ksplit != h->ksplit, near_moved = false;
   h->ksplit = ksplit;
   int rc = DE_OK;
-  if ((rc = grow(h, &h->d_abuf, &h->abuf_cap, size_t(s.batch) * h->dim, &m)) ||
-      (rc = grow(h, &h->d_rbuf, &h->rbuf_cap, size_t(ksplit) * s.batch * h->dim, &m)) ||
-      (rc = grow(h, &h->d_rloss, &h->rloss_cap, size_t(ksplit) * s.batch, &m)) ||
-      (rc = grow(h, &h->d_near_bits, &h->near_cap, size_t(s.batch) * 32, &near_moved)))
+  if ((rc = grow(h, &h->d_abuf, &h->abuf_cap, rows * h->dim, &m)) ||
+      (rc = grow(h, &h->d_rbuf, &h->rbuf_cap, ksplit * rows * h->dim, &m)) ||
+      (rc = grow(h, &h->d_rloss, &h->rloss_cap, ksplit * rows, &m)) ||
+      (rc = grow(h, &h->d_near_bits, &h->near_cap, rows * 32, &near_moved)))
     return rc;
   if (near_moved) {
     DE_CUDA(h, cudaMemsetAsync(h->d_near_bits, 0, h->near_cap * sizeof(uint32_t), h->stream));

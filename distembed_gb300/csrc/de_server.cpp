@@ -140,8 +140,8 @@ int64_t job_bytes(const de_job_spec &s) {
   if (s.precision == DE_PRECISION_BF16) {
     const int64_t kpad = std::max<int64_t>(64, (s.ns + 63) / 64 * 64);
     const int64_t parts = de::bf16_ksplit(rows, kpad);
-    b += 2 * n * D + 8 * n + (1 + parts) * B * D * 4 + parts * B * 8;  // + update rows and their losses
-    b += 2 * kpad * D * 2 + kpad * 8 + B * 32 * 4;
+    b += 2 * n * D + 8 * n + (1 + parts) * rows * D * 4 + parts * rows * 8;  // + update rows and their losses
+    b += 2 * kpad * D * 2 + kpad * 8 + rows * 32 * 4;
   } else {
     b += int64_t(de::stage_slots(batches)) * rows * D * 4;             // staging
   }

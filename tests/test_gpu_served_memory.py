@@ -29,7 +29,7 @@ def graph(n):
     return rp, col
 
 
-@pytest.mark.parametrize("dim,ns,precision", [(32, 5, "fp32"), (128, 0, "fp32")])
+@pytest.mark.parametrize("dim,ns,precision", [(32, 5, "fp32"), (128, 0, "fp32"), (128, 9, "bf16"), (256, 300, "bf16")])
 def test_minibatch_larger_than_the_graph(dim, ns, precision):
     g = graph(1000)
     whole = serve(g, dim, 2, 1000, ns, precision, 64 << 20)
