@@ -490,8 +490,9 @@ int loss_epochs(const de_handle *h, int epochs) {
 // two embeddings and writes every row of the other (d_x and the staging buffer), so an
 // epoch is one launch: no copy back, no flush, the epoch's index and rate in its
 // arguments, and the losses of many epochs summed by one launch at the end.  1,507
-// vertices, dim 32, 20 epochs with loss: 285 -> 208 us a run from host rows.
-cudaError_t enqueue_whole_graph(de_handle *h, int first_epoch, int epochs, int ns, const double *lr) {
+// vertices, dim 32, 20 epochs with loss: 285 -> 208 us a run from host rows.  ev
+// (nullable; one epoch): one event before the launch and one before what ends the run.
+cudaError_t enqueue_whole_graph(de_handle *h, int first_epoch, int epochs, int ns, const double *lr, cudaEvent_t *ev) {
   const Schedule &s = h->sched;
   PlainBatchArgs a = plain_args(h, ns);
   a.items = s.d_items;
@@ -508,7 +509,9 @@ cudaError_t enqueue_whole_graph(de_handle *h, int first_epoch, int epochs, int n
     a.epoch_at = e;
     a.lr_at = float(lr[e]);
     a.loss_off = int64_t(e % keep) * s.n_items;
-    err = launch_plain_batch(h->dim, a, item_teams(h, a), h->opt.pdl != 0, h->stream);
+    if (ev) cudaEventRecord(ev[0], h->stream);
+    err = launch_plain_batch(h->dim, a, item_teams(h, a), h->opt.pdl && !ev, h->stream);
+    if (ev) cudaEventRecord(ev[1], h->stream);
     std::swap(from, to);
     if (err == cudaSuccess && h->opt.compute_loss && (e % keep == keep - 1 || e == epochs - 1))
       err = launch_epoch_losses(h->d_loss_partial, s.n_items, e % keep + 1, h->d_block_sums, h->d_loss + (e - e % keep),
@@ -575,6 +578,9 @@ std::vector<int> epoch_launch_kinds(const de_handle *h) {
   k.push_back(3);
   return k;
 }
+
+// The form that de_run_from takes for the minibatch size prepared.
+bool whole_graph(const de_handle *h) { return h->opt.precision == DE_PRECISION_FP32 && h->sched.batches == 1; }
 
 cudaError_t enqueue_epoch(de_handle *h, int ns, cudaStream_t st, cudaEvent_t *ev) {
   return h->opt.precision == DE_PRECISION_BF16 ? enqueue_epoch_bf16(h, ns, st, ev)
@@ -1016,8 +1022,8 @@ int de_run_from(de_handle *h, int32_t first_epoch, int32_t epochs, int32_t batch
   int rc = prepare_run(h, first_epoch, epochs, batch_size, ns, lr_per_epoch);
   if (rc) return rc;
   const Schedule &s = h->sched;
-  if (h->opt.precision == DE_PRECISION_FP32 && s.batches == 1) {
-    DE_CUDA(h, enqueue_whole_graph(h, first_epoch, epochs, ns, lr_per_epoch));
+  if (whole_graph(h)) {
+    DE_CUDA(h, enqueue_whole_graph(h, first_epoch, epochs, ns, lr_per_epoch, nullptr));
   } else if (h->opt.precision == DE_PRECISION_FP32 && s.batches <= kDirectBatches) {
     for (int i = 0; i < epochs; ++i) DE_CUDA(h, enqueue_epoch(h, ns, h->stream, nullptr));
   } else {
@@ -1325,7 +1331,8 @@ int de_profile_epoch(de_handle *h, int32_t first_epoch, int32_t batch_size, int3
   if (!launch_ms || !launch_kind || capacity < n) return fail(h, DE_ERR_INVALID, "capacity below the launch count");
   std::vector<cudaEvent_t> ev(n + 1, nullptr);
   for (auto &e : ev) DE_CUDA(h, cudaEventCreate(&e));
-  cudaError_t err = enqueue_epoch(h, ns, h->stream, ev.data());
+  cudaError_t err = whole_graph(h) ? enqueue_whole_graph(h, first_epoch, 1, ns, &lr, ev.data())
+                                   : enqueue_epoch(h, ns, h->stream, ev.data());
   if (err == cudaSuccess) err = cudaEventRecord(ev[n], h->stream);
   if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
   for (int i = 0; err == cudaSuccess && i < n; ++i) {

@@ -109,6 +109,8 @@ int de_run_from(de_handle *h, int32_t first_epoch, int32_t epochs, int32_t batch
  * 1: BF16 repulsion GEMM kernel, 2: BF16 update with the exact close pairs,
  * 3: epoch flush, 4: BF16 negative gather); the launches of the profiled epoch
  * run one after another (the BF16 attractive pass and GEMMs are not overlapped).
+ * Where the minibatch is the whole graph the flush is what ends such a run: the
+ * loss's sum and the copy of the new rows into their place.
  * *count receives the number of launches; capacity must be at least that.  The
  * epoch is a real step: the embedding is updated.  No reference counterpart:
  * this is the per-kernel timing used by the benchmark. */
