@@ -641,10 +641,28 @@ int check_rowptr(de_handle *h, int64_t n, const int64_t *rowptr, int64_t nnz) {
 int bad_column(de_handle *h) { return fail(h, DE_ERR_INVALID, "column index out of range"); }
 
 // Columns to int32 on the GPU, checked against n and the edges into n-1 counted on the
-// way: the host's three passes over a million entries took longer than a small job's
-// training.  The int64 columns go through d_x, which the caller clears afterwards, in
-// as many pieces as it holds.  counters: two words of device memory.
-int upload_columns(de_handle *h, const int64_t *col, unsigned long long *counters) {
+// way: the host's passes over a million entries took longer than a small job's training.
+// The int64 columns go through d_x, which the caller clears afterwards, in as many pieces
+// as it holds.  counters: two words of device memory.  Up to kHostColumns entries, where
+// the kernel and the wait for its counts take longer (16 to 500 vertices: 0.50 ms a handle
+// against 0.47), the host does it in one pass, into `narrow`, which the stream may still
+// read when the call returns.
+constexpr int64_t kHostColumns = 32768;
+int upload_columns(de_handle *h, const int64_t *col, unsigned long long *counters, std::vector<int32_t> &narrow) {
+  if (h->nnz <= kHostColumns) {
+    narrow.resize(size_t(h->nnz));
+    int64_t bad = 0, last = 0;
+    for (int64_t q = 0; q < h->nnz; ++q) {
+      const int64_t c = col[q];
+      narrow[q] = int32_t(c);
+      bad += c < 0 || c >= h->n;
+      last += c == h->n - 1;
+    }
+    if (bad) return bad_column(h);
+    h->edges_into_last = last;
+    DE_CUDA(h, cudaMemcpyAsync(h->d_col, narrow.data(), size_t(h->nnz) * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
+    return DE_OK;
+  }
   const int64_t room = h->n * h->dim / 2;  // int64 values d_x holds
   DE_CUDA(h, cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), h->stream));
   for (int64_t off = 0; off < h->nnz; off += room) {
@@ -745,7 +763,8 @@ int create_handle(int64_t n, const int64_t *rowptr, const int64_t *col, int64_t 
   // legacy stream, and a synchronous cudaMemcpy from pageable memory may return
   // before its DMA has landed
   cudaStream_t st = h->stream;
-  if (int rc = upload_columns(h.get(), col, reinterpret_cast<unsigned long long *>(h->d_block_sums))) return bail(rc);
+  std::vector<int32_t> narrow;
+  if (int rc = upload_columns(h.get(), col, reinterpret_cast<unsigned long long *>(h->d_block_sums), narrow)) return bail(rc);
   if ((e = cudaMemcpyAsync(h->d_rowptr, rp32.data(), (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
       (e = cudaMemsetAsync(h->d_x, 0, size_t(n) * dim * sizeof(float), st)) != cudaSuccess ||
       (e = cudaMemsetAsync(h->d_done, 0, sizeof(int32_t), st)) != cudaSuccess ||
