@@ -27,6 +27,7 @@ struct de_csr {
   int64_t rows = 0, cols = 0, nnz = 0;
   int32_t device = 0;
   int64_t *d_rowptr = nullptr, *d_col = nullptr;  // one allocation, d_rowptr first
+  cudaStream_t st = nullptr;                      // the one it was built on, for its copies out
 };
 
 namespace de {
@@ -208,7 +209,9 @@ int build_on_gpu(int32_t device, int64_t rows, int64_t cols, const Entries &in, 
   out->nnz = m;
   out->d_rowptr = d_rowptr;
   out->d_col = d_col;
-  b.result = nullptr;  // the CSR's now
+  out->st = b.st;
+  b.result = nullptr;  // the CSR's now, with the stream
+  b.st = nullptr;
   return DE_OK;
 }
 
@@ -310,18 +313,13 @@ int de_csr_copy(const de_csr *c, int64_t *rowptr, int64_t *col) {
   int before = 0;
   if (cudaGetDevice(&before) != cudaSuccess || cudaSetDevice(c->device) != cudaSuccess)
     return de::csr_fail(DE_ERR_CUDA, "CSR copy: no device");
-  cudaStream_t st = nullptr;
-  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (e == cudaSuccess) {
-    de::touch_pages(col, size_t(c->nnz) * sizeof(int64_t));
-    de::touch_pages(rowptr, size_t(c->rows + 1) * sizeof(int64_t));
-    e = cudaMemcpyAsync(col, c->d_col, size_t(c->nnz) * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(rowptr, c->d_rowptr, size_t(c->rows + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = e2;
-    cudaStreamDestroy(st);
-  }
+  de::touch_pages(col, size_t(c->nnz) * sizeof(int64_t));
+  de::touch_pages(rowptr, size_t(c->rows + 1) * sizeof(int64_t));
+  cudaError_t e = cudaMemcpyAsync(col, c->d_col, size_t(c->nnz) * sizeof(int64_t), cudaMemcpyDeviceToHost, c->st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(rowptr, c->d_rowptr, size_t(c->rows + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, c->st);
+  const cudaError_t e2 = cudaStreamSynchronize(c->st);
+  if (e == cudaSuccess) e = e2;
   cudaSetDevice(before);
   if (e != cudaSuccess) return de::csr_fail(DE_ERR_CUDA, std::string("CSR copy: ") + cudaGetErrorString(e));
   return DE_OK;
@@ -334,6 +332,7 @@ void de_csr_free(de_csr *c) {
     const bool known = cudaGetDevice(&before) == cudaSuccess;
     cudaSetDevice(c->device);
     cudaFree(c->d_rowptr);
+    cudaStreamDestroy(c->st);
     if (known) cudaSetDevice(before);
   }
   delete c;
