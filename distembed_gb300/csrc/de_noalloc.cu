@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(W * 32) noalloc_rows_kernel(const NoAllocArgs 
   de::dev::pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = blockIdx.x, row = a.base + r;
-  const int e0 = a.rowptr[row], deg = a.rowptr[row + 1] - e0;
+  const int e0 = a.rowptr[row], deg = max(a.rowptr[row + 1] - e0, 0);  // a pointer that falls: no entries
   de::dev::Frag<D> xi, acc;
   nload<D, kWide>(xi, a.x + size_t(row) * D, lane);
   acc.zero();
