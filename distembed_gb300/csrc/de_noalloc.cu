@@ -131,7 +131,7 @@ __device__ __forceinline__ void nforces(const NoAllocArgs &a, de::dev::Frag<D> &
 // One row per CTA of W warps: the row's CSR entries and then its negatives in
 // groups of U, group q on warp q % W; the warps' sums are added in warp order.
 // A minibatch is too small to fill the GPU with bytes, so a call takes as long as
-// the longest chain of dependent loads.  Here a row of up to 8 W pairs is one
+// the longest chain of dependent loads.  Here a row of up to U W pairs is one
 // round: row pointer, column ids, rows.  Measured on the epoch of a 2,000-vertex
 // kNN graph (8 calls of 256 rows of about 14 neighbours, dim 64, 5 negatives):
 // 305 us with a warp per row and one neighbour in flight, 56 us so (7 us a call, both
@@ -239,14 +239,20 @@ cudaError_t nlaunch(void (*k)(P...), int grid, int block, cudaStream_t s, A... a
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
-// Eight warps a row where the rows then still fit the GPU at once (152 SMs x 8
-// CTAs of 256 threads), so that the longest rows finish sooner; four beyond.
-constexpr int kWideTeamRows = 152 * 8;
+// Eight warps a row, so that the longest rows finish sooner, where every row's CTA then
+// still is resident (the registers of 256 threads: six CTAs an SM at dim 32, five at 64,
+// three at 128 and 256); four warps beyond.  Time of a call with four warps over that with
+// eight, rows of about 14 / 40 entries: dim 256, 128 rows 1.00 / 1.23, 456 1.01 / 1.21, 912
+// 0.93 / 0.93, 1216 0.93 / 0.96; dim 128, 456 rows 0.99 / 1.03, 912 0.92 / 0.91, 1216 0.82 /
+// 0.96, 2432 0.70 / 0.89; dim 64, 760 rows 1.01 / 0.99, 1216 0.96 / 0.96, 2432 0.82 / 0.96;
+// dim 32, 912 rows 0.99 / 1.03, 1216 0.98 / 0.90, 2432 0.88 / 0.97.
+template <int D>
+constexpr int kWideTeamRows = 152 * (D == 32 ? 6 : D == 64 ? 5 : 3);
 
 template <int D, bool kWide>
 cudaError_t nrun(const NoAllocArgs &a, cudaStream_t s) {
   constexpr int U = D == 256 ? 4 : 8;
-  cudaError_t e = a.rows <= kWideTeamRows ? nlaunch(noalloc_rows_kernel<D, U, 8, kWide>, a.rows, 256, s, a)
+  cudaError_t e = a.rows <= kWideTeamRows<D> ? nlaunch(noalloc_rows_kernel<D, U, 8, kWide>, a.rows, 256, s, a)
                                           : nlaunch(noalloc_rows_kernel<D, U, 4, kWide>, a.rows, 128, s, a);
   if (e != cudaSuccess) return e;
   const int64_t total = int64_t(a.rows) * D, per = 256 * (kWide ? 4 : 1);
