@@ -531,7 +531,6 @@ cudaError_t launch_plain_batch(int dim, const PlainBatchArgs &a, bool teams, boo
   const int team_grid = (a.n_items * w + kPlainWarps - 1) / kPlainWarps;
   if (w == 4) {
     switch (dim) {
-      case 32: return launch(plain_team_kernel<32, 4>, team_grid, block, a, pdl, s);
       case 64: return launch(plain_team_kernel<64, 4>, team_grid, block, a, pdl, s);
       case 128: return launch(plain_team_kernel<128, 4>, team_grid, block, a, pdl, s);
       case 256: return launch(plain_team_kernel<256, 4>, team_grid, block, a, pdl, s);
