@@ -338,8 +338,8 @@ int de_mm_read_gpu(const char *path, int32_t device, de_csr **out);
 int de_coo_to_csr(int64_t rows, int64_t cols, const int64_t *row_idx, const int64_t *col_idx, int64_t nnz,
                   int32_t mirror, int32_t device, de_csr **out);
 int de_csr_info(const de_csr *c, int64_t *rows, int64_t *cols, int64_t *nnz);
-/* Copies the CSR, which stays on the GPU until de_csr_free, to host arrays
- * rowptr[rows + 1] and col[nnz]. */
+/* Copies the CSR, which stays on the GPU (8 bytes a row and an entry) until de_csr_free,
+ * to host arrays rowptr[rows + 1] and col[nnz]; an error of the copy is returned. */
 int de_csr_copy(const de_csr *c, int64_t *rowptr, int64_t *col);
 void de_csr_free(de_csr *c);
 /* Embedding writer of ParallelIO::parallel_write (cpp/io/parrallel_IO.hpp:90-146):
@@ -375,7 +375,8 @@ int de_spmm_f32(de_handle *h, int32_t batch_size, float lr, float *y, int32_t on
  *     pruned to their k largest values after every iteration but the last.
  * At equal values the pruning drops the lower dim first (the reference's heap
  * order at ties is its own).  The handle's FP32 embedding becomes the rows'
- * FP32 mirror (0 for an absent entry).  FP32 handles, dim 32, 64, 128 or 256. */
+ * FP32 mirror (0 for an absent entry).  FP32 handles, dim 32, 64, 128 or 256.
+ * After an error x may hold its values, the new rows or some of each. */
 int de_sparse_embedding(de_handle *h, double *x, int32_t iterations, int32_t batch_size, int32_t ns, double lr,
                         double density, int32_t merge, double *coll);
 /* The same in three steps, the rows kept on the device between them:
