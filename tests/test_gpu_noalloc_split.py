@@ -23,9 +23,12 @@ RESIDENT = {32: 152 * 6, 64: 152 * 5, 128: 152 * 3, 256: 152 * 3}
 def _built():
     from distembed_gb300 import build
     build.build()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]):  # its first session sees nothing
-        torch.zeros(1, device="cuda")
-        torch.cuda.synchronize()
+    for _ in range(5):  # the profiler's first session in a process may see nothing
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+            torch.zeros(1, device="cuda").add_(1)
+            torch.cuda.synchronize()
+        if any(e.device_type == torch.autograd.DeviceType.CUDA for e in p.events()):
+            break
 
 
 @pytest.mark.parametrize("shift", [0, 4])

@@ -18,9 +18,12 @@ def _built():
 
 @pytest.fixture(scope="module", autouse=True)
 def _profiler(_built):
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]):  # its first session sees nothing
-        torch.zeros(1, device="cuda")
-        torch.cuda.synchronize()
+    for _ in range(5):  # the profiler's first session in a process may see nothing
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+            torch.zeros(1, device="cuda").add_(1)
+            torch.cuda.synchronize()
+        if any(e.device_type == torch.autograd.DeviceType.CUDA for e in p.events()):
+            break
 
 
 def kernels(f):

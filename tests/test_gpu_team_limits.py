@@ -25,9 +25,12 @@ CASES = [(dim, items + more, 4 if items + more <= four else 2 if items + more <=
 def _built():
     from distembed_gb300 import build
     build.build()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]):  # its first session sees nothing
-        torch.zeros(1, device="cuda")
-        torch.cuda.synchronize()
+    for _ in range(5):  # the profiler's first session in a process may see nothing
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+            torch.zeros(1, device="cuda").add_(1)
+            torch.cuda.synchronize()
+        if any(e.device_type == torch.autograd.DeviceType.CUDA for e in p.events()):
+            break
 
 
 def graph(n, rows, seed):
